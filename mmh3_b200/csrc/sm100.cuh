@@ -133,6 +133,14 @@ __device__ __forceinline__ void tma_load_3d(uint32_t destination, const CUtensor
                  : "memory");
 }
 
+__device__ __forceinline__ void tma_load_4d(uint32_t destination, const CUtensorMap *map,
+                                            uint32_t bar, int c0, int c1, int c2, int c3) {
+    asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes "
+                 "[%0], [%1, {%3, %4, %5, %6}], [%2];" ::"r"(destination),
+                 "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
+                 : "memory");
+}
+
 // A hint: the 128-byte line holding `address` into L1.
 __device__ __forceinline__ void prefetch_l1(const void *address) {
     asm volatile("prefetch.global.L1 [%0];" ::"l"(address));

@@ -186,6 +186,64 @@ def test_grouped_heads_and_batches(oracle):
     assert torch.max(torch.abs(output.cpu().double() - expected)) <= 2e-2
 
 
+@pytest.mark.parametrize("element_type,head_dim,tokens,batch,causal,order", [
+    (0, 128, 130, 3, 1, "items"),       # [batch, tokens, heads, dim]
+    (1, 64, 257, 9, 0, "items"),
+    (1, 64, 300, 2, 0, "tokens"),       # [tokens, batch, heads, dim]
+    (0, 128, 1, 4, 0, "heads"),         # [heads, batch, tokens, dim]
+    (0, 64, 140, 3, 0, "shared"),       # one key and value for all items: a stride of zero
+    (0, 128, 140, 3, 0, "off grid"),    # items that do not start on 16 bytes
+    (1, 128, 40, 3, 0, "overlapping"),  # outputs that the next item partly writes over
+])
+@pytest.mark.parametrize("rope", [False, True])
+def test_a_batch_equals_its_items(element_type, head_dim, tokens, batch, causal, order, rope):
+    """A batch that TMA can describe goes in one launch, the others item by item: the same bits as
+    one call per item, in order, either way."""
+    heads, group = 4, 2
+    dtype = torch.float16 if element_type == 1 else torch.bfloat16
+    generator = torch.Generator().manual_seed(tokens + batch)
+    pairs = 20
+    angles = (torch.rand((tokens, pairs), generator=generator) * 6.0 - 3.0).cuda()
+
+    def strides(count):
+        if order == "tokens":
+            return batch * count * head_dim, head_dim, count * head_dim
+        if order == "heads":
+            return head_dim, batch * tokens * head_dim, tokens * head_dim
+        return count * head_dim, head_dim, tokens * count * head_dim
+
+    counts = (heads, heads // group, heads // group, heads)
+    layout = [list(strides(count)) for count in counts]
+    if order == "shared":
+        layout[1][2] = layout[2][2] = 0
+    if order == "off grid":
+        for operand in layout:
+            operand[2] += 4
+    if order == "overlapping":
+        layout[3][2] //= 2
+    sizes = [1 + (tokens - 1) * t + (count - 1) * h + (batch - 1) * b + head_dim
+             for (t, h, b), count in zip(layout, counts)]
+    query, key, value = (torch.randn(size, generator=generator).to(dtype).cuda()
+                         for size in sizes[:3])
+
+    def run(whole):
+        output = torch.zeros(sizes[3], dtype=dtype, device="cuda")
+        operands = (query, key, value, output)
+        described = attention.make_layout(*zip(*layout), heads_per_key_value=group, causal=causal)
+        for item in range(1 if whole else batch):
+            views = [tensor[item * operand[2]:] for tensor, operand in zip(operands, layout)]
+            arguments = (element_type, head_dim, *views, tokens, heads, batch if whole else 1,
+                         described, SCALE)
+            if rope:
+                attention.attention_roped(*arguments, angles, pairs, 1e-6)
+            else:
+                attention.attention(*arguments)
+        assert attention.take_status() == 0
+        return output
+
+    assert torch.equal(run(True).view(torch.int16), run(False).view(torch.int16))
+
+
 def reference_attention(q, k, v, group, causal):
     """softmax(q k^T * scale) v in float64 with torch, [batch, tokens, heads, 128] operands."""
     keys = k.double().repeat_interleave(group, dim=2)
