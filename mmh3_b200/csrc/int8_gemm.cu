@@ -10,22 +10,31 @@
 // crates/mmh3-cuda/kernels/int8_gemm.cu:321-591 (mma.sync over a two-stage ring) and keeps its
 // arithmetic: the integer sums are exact, and the FP32 operations after them are the
 // same in the same order, so without an adapter the outputs and the column maxima are the same
-// bits. With an adapter a tile is 128 rows: its INT32 accumulator and an FP32 accumulator for
-// down . up^T sit side by side in tensor memory, and after the K blocks the ring carries blocks of
-// 64 ranks of the two BF16 operands, in the same 128-byte rows, for kind::f16 MMAs. Those sums
-// come in the tensor cores' own order, so that result is held to the reference's bounds instead.
+// bits. With an adapter the INT32 accumulator of a tile and an FP32 accumulator for down . up^T sit
+// side by side in tensor memory, and after the K blocks the ring carries blocks of 64 ranks of the
+// two BF16 operands, in the same 128-byte rows, for kind::f16 MMAs. Those sums come in the tensor
+// cores' own order, so that result is held to the reference's bounds instead.
 //
-// One persistent CTA per SM walks tiles of 256 rows by 256 columns in bands of rows of tiles, so
-// the CTAs in flight share rows of activations and columns of weights in L2. A tile is two
-// accumulators of 128 rows by 256 columns of INT32 in tensor memory (all 512 columns of the SM).
-// Warp 0 streams stages of 128 bytes of K (32 KB of activations, 32 KB of weights, 128-byte
-// swizzle) through a ring of three with TMA; one thread of warp 1 issues tcgen05.mma kind::i8 of
-// 128 x 256 x 32 from shared memory; eight warps scale and round the accumulators, turn their rows
-// around in a staging tile of shared memory so that the stores cover whole 128-byte runs, and give
-// tensor memory back as soon as the last columns are in registers, while the ring fills for the
-// next tile. At this tile shape a stage of 64 KB feeds 1,024 cycles of MMA, 64 bytes a cycle,
-// which is what an SM can take from L2; a tile of 128 x 256 would leave room for a second pair of
-// accumulators and an epilogue hidden behind the next tile's MMAs, but needs 96 bytes a cycle.
+// A persistent pair of CTAs (a cluster of two, one CTA per SM) walks tiles of 256 rows by 256
+// columns in bands of rows of tiles, so the pairs in flight share rows of activations and columns
+// of weights in L2. Each CTA keeps 128 rows of the tile: INT32 accumulators of 128 x 256 in its
+// tensor memory, two of them, which take turns from tile to tile, so that the MMAs of a tile run
+// while the last one is scaled and stored. Warp 0 of each CTA streams its 128 rows of activations
+// and its half of the weights' 256 columns, 128 bytes of K at a time (32 KB, 128-byte swizzle),
+// through a ring of six with TMA; one thread of warp 1 of the first CTA issues tcgen05.mma
+// cta_group::2 kind::i8 of 256 x 256 x 32 over both CTAs' shared memory; eight warps of each CTA
+// scale and round its accumulator, turn their rows around in a staging tile of shared memory so
+// that the stores cover whole 128-byte runs, and give the accumulator back as soon as its last
+// columns are in registers.
+//
+// What bounds it is the MMAs and, in a long run, the power they draw. The pair is what hides the
+// epilogue: an SM takes 32 KB per 512 cycles of MMA from L2, 64 bytes a cycle, about what it can
+// get; one CTA alone with 128 x 256 tiles and two accumulators would need 96, and with tiles of 256
+// x 256 (64 bytes a cycle, no second accumulator) the tensor cores waited for an epilogue of about
+// 12,000 cycles in every 46,000. Against that kernel, whole calls: a SwiGLU layer of 4,213 x 28,672
+// x 5,376 with an adapter of rank 384 went from 710 us to 672 (an adapter leaves no room for the
+// second accumulator, but its 128-row tiles took the 96 bytes a cycle), a DiT attention layer of
+// 16,896 tokens, whose qkv projection is a fifth of it, from 7.70 ms to 7.52.
 #include "common.cuh"
 #include "sm100.cuh"
 
@@ -36,28 +45,20 @@ namespace {
 
 using namespace sm100;
 
-constexpr int TILE_M = 128;     // rows of one accumulator
+constexpr int TILE_M = 128;     // rows of a tile in one CTA of the pair
+constexpr int PAIR_M = 2 * TILE_M;
 constexpr int TILE_N = 256;
 constexpr int BLOCK_K = 128;    // bytes of one stage along K: 128 INT8 values, 64 BF16 ranks
-constexpr int COLUMNS_BYTES = TILE_N * BLOCK_K;
+constexpr int ROWS_BYTES = TILE_M * BLOCK_K;
+constexpr int COLUMNS_BYTES = TILE_N / 2 * BLOCK_K; // the half of the tile's columns a CTA loads
+constexpr int STAGE_BYTES = ROWS_BYTES + COLUMNS_BYTES;
+constexpr int STAGES = 6;
 // Where an epilogue warp turns its 32 rows of 64 columns around for the stores.
 constexpr int STAGING_ROW = 128;
 constexpr int STAGING_BYTES = 32 * STAGING_ROW;
 constexpr int EPILOGUE_WARPS = 8;
-constexpr int MAX_STAGES = 4;
-
-// Without a low-rank adapter a tile is 256 rows: two INT32 accumulators fill tensor memory. With
-// one it is 128 rows: one INT32 accumulator, and one FP32 accumulator for down . up^T beside it.
-template <bool ADAPTED> struct Shape {
-    static constexpr int ROW_TILES = ADAPTED ? 1 : 2;
-    static constexpr int STAGES = ADAPTED ? 4 : 3;
-    static constexpr int ROWS_BYTES = ROW_TILES * TILE_M * BLOCK_K;
-    static constexpr int STAGE_BYTES = ROWS_BYTES + COLUMNS_BYTES;
-    static constexpr int SMEM_BYTES =
-        STAGES * STAGE_BYTES + EPILOGUE_WARPS * STAGING_BYTES + 1024;
-    static_assert(STAGES <= MAX_STAGES, "more stages than barriers");
-    static_assert(SMEM_BYTES + 256 <= 227 * 1024, "ring, staging and barriers exceed an SM");
-};
+constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + EPILOGUE_WARPS * STAGING_BYTES + 1024;
+static_assert(SMEM_BYTES + 256 <= 227 * 1024, "ring, staging and barriers exceed an SM");
 
 constexpr int LOAD_WARP = 0;
 constexpr int MMA_WARP = 1;
@@ -71,17 +72,17 @@ constexpr unsigned int STATUS_GEMM = 0x00040000u;
 
 enum Barrier {
     RING_FULL = 0,
-    RING_EMPTY = RING_FULL + MAX_STAGES,
-    ACCUMULATOR_FULL = RING_EMPTY + MAX_STAGES,
-    ACCUMULATOR_EMPTY,
-    BARRIERS,
+    RING_EMPTY = RING_FULL + STAGES,
+    ACCUMULATOR_FULL = RING_EMPTY + STAGES, // one per accumulator
+    ACCUMULATOR_EMPTY = ACCUMULATOR_FULL + 2,
+    BARRIERS = ACCUMULATOR_EMPTY + 2,
 };
 
 constexpr uint32_t PRODUCT_MMA =
-    instruction_descriptor(ACCUMULATE_S32, FORMAT_S8, FORMAT_S8, 0, 0, TILE_M, TILE_N);
+    instruction_descriptor(ACCUMULATE_S32, FORMAT_S8, FORMAT_S8, 0, 0, PAIR_M, TILE_N);
 
 constexpr uint32_t ADAPTER_MMA =
-    instruction_descriptor(ACCUMULATE_F32, FORMAT_BF16, FORMAT_BF16, 0, 0, TILE_M, TILE_N);
+    instruction_descriptor(ACCUMULATE_F32, FORMAT_BF16, FORMAT_BF16, 0, 0, PAIR_M, TILE_N);
 
 struct GemmMaps {
     CUtensorMap activations;  // [m, k] INT8
@@ -137,17 +138,16 @@ __device__ __forceinline__ uint32_t gated_pair(Output *output, uint32_t gate_wor
 }
 
 template <typename Output, bool SWIGLU, bool ADAPTED>
-__global__ void __launch_bounds__(THREADS, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
     int8_gemm_kernel(const __grid_constant__ GemmMaps maps,
                      const float *__restrict__ activation_scales,
                      const float *__restrict__ weight_scales, const float *__restrict__ bias,
                      Output *__restrict__ output, int m, int n, int k_blocks, int output_stride,
                      TileWalk walk, unsigned *maxima, int maxima_first_column,
                      int adapter_blocks, float adapter_scale, unsigned int *status) {
-    constexpr int ROW_TILES = Shape<ADAPTED>::ROW_TILES;
-    constexpr int STAGES = Shape<ADAPTED>::STAGES;
-    constexpr int ROWS_BYTES = Shape<ADAPTED>::ROWS_BYTES;
-    constexpr int STAGE_BYTES = Shape<ADAPTED>::STAGE_BYTES;
+    // Accumulators of 256 columns that take turns from tile to tile: the adapter's sum takes the
+    // second one's columns.
+    constexpr int ACCUMULATORS = ADAPTED ? 1 : 2;
     extern __shared__ uint8_t shared_raw[];
     __shared__ __align__(8) uint64_t barriers[BARRIERS];
     __shared__ uint32_t tmem_slot_storage;
@@ -160,23 +160,29 @@ __global__ void __launch_bounds__(THREADS, 1)
     const int warp = warp_index();
     const int lane = threadIdx.x % 32;
     const int tiles = walk.tiles();
+    const int rank = static_cast<int>(cluster_rank()); // the CTA of the pair; the first issues the MMAs
+    const int first_tile = blockIdx.x / 2;
+    const int tile_step = gridDim.x / 2;
 
     if (threadIdx.x == 0) {
         for (int stage = 0; stage < STAGES; stage++) {
             mbar_init(barrier(RING_FULL + stage), 1);
             mbar_init(barrier(RING_EMPTY + stage), 1);
         }
-        mbar_init(barrier(ACCUMULATOR_FULL), 1);
-        mbar_init(barrier(ACCUMULATOR_EMPTY), EPILOGUE_WARPS);
+        for (int buffer = 0; buffer < ACCUMULATORS; buffer++) {
+            mbar_init(barrier(ACCUMULATOR_FULL + buffer), 1);
+            mbar_init(barrier(ACCUMULATOR_EMPTY + buffer), 2 * EPILOGUE_WARPS);
+        }
         *abort_flag = 0;
         fence_barrier_init();
         fence_proxy_async();
     }
     if (warp == MMA_WARP) {
-        tmem_alloc(smem_u32(const_cast<uint32_t *>(tmem_slot)), TMEM_COLUMNS);
+        tmem_alloc_pair(smem_u32(const_cast<uint32_t *>(tmem_slot)), TMEM_COLUMNS);
     }
     tcgen05_fence_before();
     __syncthreads();
+    cluster_sync();
     tcgen05_fence_after();
     const uint32_t tmem = *tmem_slot;
 
@@ -190,11 +196,14 @@ __global__ void __launch_bounds__(THREADS, 1)
             }
             int item = 0;
             bool alive = true;
-            for (int tile = blockIdx.x; alive && tile < tiles; tile += gridDim.x) {
+            for (int tile = first_tile; alive && tile < tiles; tile += tile_step) {
                 int tile_m, tile_n;
                 walk.locate(tile, tile_m, tile_n);
+                const int row = tile_m * PAIR_M + rank * TILE_M;
+                const int column = tile_n * TILE_N + rank * (TILE_N / 2);
                 // The K blocks of the INT8 operands, then the adapter's blocks of 64 ranks: the
-                // same 128-byte rows in the same places.
+                // same 128-byte rows in the same places. The bytes of both CTAs are counted by the
+                // first one's barrier, which expects them all.
                 for (int block = 0; block < k_blocks + adapter_blocks; block++, item++) {
                     const int stage = item % STAGES;
                     const int use = item / STAGES;
@@ -204,57 +213,68 @@ __global__ void __launch_bounds__(THREADS, 1)
                         break;
                     }
                     const uint32_t destination = base + stage * STAGE_BYTES;
+                    const uint32_t full = cluster_address(barrier(RING_FULL + stage), 0);
                     const bool adapter = block >= k_blocks;
                     // Coordinates are in elements: bytes for INT8, BF16 values for the adapter.
                     const int along = adapter ? (block - k_blocks) * (BLOCK_K / 2) : block * BLOCK_K;
-                    mbar_expect_tx(barrier(RING_FULL + stage), STAGE_BYTES);
-                    tma_load_2d(destination, adapter ? &maps.adapter_down : &maps.activations,
-                                barrier(RING_FULL + stage), along, tile_m * (ROW_TILES * TILE_M));
-                    tma_load_2d(destination + ROWS_BYTES,
-                                adapter ? &maps.adapter_up : &maps.weights,
-                                barrier(RING_FULL + stage), along, tile_n * TILE_N);
+                    if (rank == 0) {
+                        mbar_expect_tx(barrier(RING_FULL + stage), 2 * STAGE_BYTES);
+                    }
+                    tma_load_2d_pair(destination,
+                                     adapter ? &maps.adapter_down : &maps.activations, full, along,
+                                     row);
+                    tma_load_2d_pair(destination + ROWS_BYTES,
+                                     adapter ? &maps.adapter_up : &maps.weights, full, along,
+                                     column);
                 }
+            }
+            // The commits of the last uses arrive here from the first CTA: they do before this CTA
+            // may leave.
+            for (int last = item - 1; alive && last >= 0 && last >= item - STAGES; last--) {
+                alive = mbar_wait(barrier(RING_EMPTY + last % STAGES), last / STAGES & 1, watchdog,
+                                  STATUS_GEMM | 5);
             }
         }
     } else if (warp == MMA_WARP) {
-        if (elect_one()) {
-            // The MMAs of one accumulator over one stage: four steps of 32 along K.
-            auto multiply = [&](int half, int stage, bool first) {
+        if (rank == 0 && elect_one()) {
+            // The MMAs of one stage, both CTAs' halves: four steps of 32 INT8 values along K into
+            // `accumulator`, or of 16 BF16 ranks into the adapter's.
+            auto multiply = [&](uint32_t accumulator, int stage, bool first) {
                 const uint32_t stage_base = base + stage * STAGE_BYTES;
-                const uint64_t rows =
-                    smem_descriptor(stage_base + half * (TILE_M * BLOCK_K), 16, 1024);
+                const uint64_t rows = smem_descriptor(stage_base, 16, 1024);
                 const uint64_t columns = smem_descriptor(stage_base + ROWS_BYTES, 16, 1024);
                 #pragma unroll
                 for (int step = 0; step < BLOCK_K / 32; step++) {
-                    mma_i8_ss(tmem + half * TILE_N, advance_descriptor(rows, step * 32),
-                              advance_descriptor(columns, step * 32), PRODUCT_MMA,
-                              !first || step > 0);
+                    mma_i8_pair_ss(accumulator, advance_descriptor(rows, step * 32),
+                                   advance_descriptor(columns, step * 32), PRODUCT_MMA,
+                                   !first || step > 0);
                 }
             };
-            // down . up^T over one stage of 64 ranks: four steps of 16 BF16 values along K.
             auto adapt = [&](int stage, bool first) {
                 const uint32_t stage_base = base + stage * STAGE_BYTES;
                 const uint64_t rows = smem_descriptor(stage_base, 16, 1024);
                 const uint64_t columns = smem_descriptor(stage_base + ROWS_BYTES, 16, 1024);
                 #pragma unroll
                 for (int step = 0; step < BLOCK_K / 32; step++) {
-                    mma_f16_ss(tmem + TMEM_ADAPTER, advance_descriptor(rows, step * 32),
-                               advance_descriptor(columns, step * 32), ADAPTER_MMA,
-                               !first || step > 0);
+                    mma_f16_pair_ss(tmem + TMEM_ADAPTER, advance_descriptor(rows, step * 32),
+                                    advance_descriptor(columns, step * 32), ADAPTER_MMA,
+                                    !first || step > 0);
                 }
             };
             int item = 0;
             int round = 0;
             bool alive = true;
-            for (int tile = blockIdx.x; alive && tile < tiles; tile += gridDim.x, round++) {
+            for (int tile = first_tile; alive && tile < tiles; tile += tile_step, round++) {
+                const int buffer = round % ACCUMULATORS;
+                const int use = round / ACCUMULATORS;
                 for (int block = 0; block < k_blocks + adapter_blocks; block++, item++) {
                     const int stage = item % STAGES;
                     alive = mbar_wait(barrier(RING_FULL + stage), (item / STAGES) & 1, watchdog,
                                       STATUS_GEMM | 2);
-                    if (alive && block == 0 && round > 0) {
-                        // The epilogue warps have read the last tile out of both accumulators.
-                        alive = mbar_wait(barrier(ACCUMULATOR_EMPTY), (round - 1) & 1, watchdog,
-                                          STATUS_GEMM | 3);
+                    if (alive && block == 0 && use > 0) {
+                        // The epilogue warps of both CTAs have read this accumulator's last tile.
+                        alive = mbar_wait(barrier(ACCUMULATOR_EMPTY + buffer), (use - 1) & 1,
+                                          watchdog, STATUS_GEMM | 3);
                     }
                     if (!alive) {
                         break;
@@ -263,15 +283,12 @@ __global__ void __launch_bounds__(THREADS, 1)
                     if (ADAPTED && block >= k_blocks) {
                         adapt(stage, block == k_blocks);
                     } else {
-                        #pragma unroll
-                        for (int half = 0; half < ROW_TILES; half++) {
-                            multiply(half, stage, block == 0);
-                        }
+                        multiply(tmem + buffer * TILE_N, stage, block == 0);
                     }
-                    tcgen05_commit(barrier(RING_EMPTY + stage));
+                    tcgen05_commit_pair(barrier(RING_EMPTY + stage));
                 }
                 if (alive) {
-                    tcgen05_commit(barrier(ACCUMULATOR_FULL));
+                    tcgen05_commit_pair(barrier(ACCUMULATOR_FULL + buffer));
                 }
             }
         }
@@ -285,9 +302,11 @@ __global__ void __launch_bounds__(THREADS, 1)
                            epilogue_warp * STAGING_BYTES;
         int round = 0;
         bool alive = true;
-        for (int tile = blockIdx.x; alive && tile < tiles; tile += gridDim.x, round++) {
+        for (int tile = first_tile; alive && tile < tiles; tile += tile_step, round++) {
+            const int buffer = round % ACCUMULATORS;
             int tile_m, tile_n;
             walk.locate(tile, tile_m, tile_n);
+            const int first_row = tile_m * PAIR_M + rank * TILE_M + quarter * 32;
             // The warp's 128 columns lie in one group of 128.
             const int first_column = tile_n * TILE_N + column_half * (TILE_N / 2);
             const bool inside = first_column < n;
@@ -301,31 +320,37 @@ __global__ void __launch_bounds__(THREADS, 1)
                     wanted = weight_scales + first_column + line * 32;
                 } else if (lane < 8 && bias != nullptr) {
                     wanted = bias + first_column + line * 32;
-                } else if (lane >= 8 && lane < 8 + ROW_TILES) {
-                    const int rows = tile_m * (ROW_TILES * TILE_M) + (lane - 8) * TILE_M +
-                                     quarter * 32;
-                    wanted = rows < m ? activation_scales + rows : nullptr;
+                } else if (lane == 8 && first_row < m) {
+                    wanted = activation_scales + first_row;
                 }
                 if (wanted != nullptr) {
                     prefetch_l1(wanted);
                 }
             }
-            alive = mbar_wait(barrier(ACCUMULATOR_FULL), round & 1, watchdog, STATUS_GEMM | 4);
+            alive = mbar_wait(barrier(ACCUMULATOR_FULL + buffer), (round / ACCUMULATORS) & 1, watchdog,
+                              STATUS_GEMM | 4);
             alive = __all_sync(0xffffffffu, alive);
             if (!alive) {
                 break;
             }
             tcgen05_fence_after();
-            auto accumulator = [&](int half, int chunk) {
-                return tmem + lane_base + half * TILE_N + column_half * (TILE_N / 2) +
+            auto accumulator = [&](int chunk) {
+                return tmem + lane_base + buffer * TILE_N + column_half * (TILE_N / 2) +
                        chunk * CHUNK;
+            };
+            auto release = [&]() {
+                tcgen05_fence_before();
+                __syncwarp();
+                if (lane == 0) {
+                    mbar_arrive_cluster(cluster_address(barrier(ACCUMULATOR_EMPTY + buffer), 0));
+                }
             };
             // Two buffers take turns: the load of the next 32 columns is in flight while these
             // are scaled. tcgen05.wait::ld waits for every load, so the next one is issued right
             // after it.
             uint32_t even[CHUNK], odd[CHUNK];
             if constexpr (!ADAPTED) {
-                tmem_load_32(accumulator(0, 0), even);
+                tmem_load_32(accumulator(0), even);
             }
             // adapter_scale * (down . up^T) joins the scaled product as the reference adds it:
             // (product / adapter_scale + down . up^T) * adapter_scale
@@ -334,168 +359,151 @@ __global__ void __launch_bounds__(THREADS, 1)
             const float2 inverse_adapter_scales =
                 make_float2(inverse_adapter_scale, inverse_adapter_scale);
             const float2 adapter_scales = make_float2(adapter_scale, adapter_scale);
-            #pragma unroll 1
-            for (int half = 0; half < ROW_TILES; half++) {
-                const int first_row =
-                    tile_m * (ROW_TILES * TILE_M) + half * TILE_M + quarter * 32;
-                const int row = first_row + lane;
-                // Nothing of these rows and columns exists: the whole warp only drains.
-                const bool idle = !inside || first_row >= m;
-                const float row_scale = row < m ? __ldg(activation_scales + row) : 0.0f;
-                const float2 row_scales = make_float2(row_scale, row_scale);
-                uint32_t magnitudes = 0;
+            const int row = first_row + lane;
+            // Nothing of these rows and columns exists: the whole warp only drains.
+            const bool idle = !inside || first_row >= m;
+            const float row_scale = row < m ? __ldg(activation_scales + row) : 0.0f;
+            const float2 row_scales = make_float2(row_scale, row_scale);
+            uint32_t magnitudes = 0;
 
-                // Scales, rounds and stages 32 columns of the lane's row.
-                auto scale = [&](const uint32_t (&products)[CHUNK],
-                                 const uint32_t (&low_rank)[CHUNK], int chunk) {
-                    const int column = first_column + chunk * CHUNK;
-                    const float2 *column_scales =
-                        reinterpret_cast<const float2 *>(weight_scales + column);
-                    const float2 *column_bias = reinterpret_cast<const float2 *>(bias + column);
-                    uint32_t words[CHUNK / 2];
+            // Scales, rounds and stages 32 columns of the lane's row.
+            auto scale = [&](const uint32_t (&products)[CHUNK],
+                             const uint32_t (&low_rank)[CHUNK], int chunk) {
+                const int column = first_column + chunk * CHUNK;
+                const float2 *column_scales =
+                    reinterpret_cast<const float2 *>(weight_scales + column);
+                const float2 *column_bias = reinterpret_cast<const float2 *>(bias + column);
+                uint32_t words[CHUNK / 2];
+                #pragma unroll
+                for (int pair = 0; pair < CHUNK / 2; pair++) {
+                    float2 scaled = make_float2(
+                        static_cast<float>(static_cast<int32_t>(products[pair * 2])),
+                        static_cast<float>(static_cast<int32_t>(products[pair * 2 + 1])));
+                    scaled = __fmul2_rn(__fmul2_rn(scaled, row_scales),
+                                        __ldg(column_scales + pair));
+                    if constexpr (ADAPTED) {
+                        const float2 added = make_float2(__uint_as_float(low_rank[pair * 2]),
+                                                         __uint_as_float(low_rank[pair * 2 + 1]));
+                        scaled = __fmul2_rn(
+                            __fadd2_rn(__fmul2_rn(scaled, inverse_adapter_scales), added),
+                            adapter_scales);
+                    }
+                    if (bias != nullptr) {
+                        scaled = __fadd2_rn(scaled, __ldg(column_bias + pair));
+                    }
+                    words[pair] = pack(output, scaled);
+                }
+                if (track && row < m) {
+                    // Magnitudes of BF16 values order like unsigned integers.
                     #pragma unroll
                     for (int pair = 0; pair < CHUNK / 2; pair++) {
-                        float2 scaled = make_float2(
-                            static_cast<float>(static_cast<int32_t>(products[pair * 2])),
-                            static_cast<float>(static_cast<int32_t>(products[pair * 2 + 1])));
-                        scaled = __fmul2_rn(__fmul2_rn(scaled, row_scales),
-                                            __ldg(column_scales + pair));
-                        if constexpr (ADAPTED) {
-                            const float2 added = make_float2(__uint_as_float(low_rank[pair * 2]),
-                                                             __uint_as_float(low_rank[pair * 2 + 1]));
-                            scaled = __fmul2_rn(
-                                __fadd2_rn(__fmul2_rn(scaled, inverse_adapter_scales), added),
-                                adapter_scales);
-                        }
-                        if (bias != nullptr) {
-                            scaled = __fadd2_rn(scaled, __ldg(column_bias + pair));
-                        }
-                        words[pair] = pack(output, scaled);
-                    }
-                    if (track && row < m) {
-                        // Magnitudes of BF16 values order like unsigned integers.
-                        #pragma unroll
-                        for (int pair = 0; pair < CHUNK / 2; pair++) {
-                            magnitudes = __vmaxu2(magnitudes, words[pair] & 0x7fff7fffu);
-                        }
-                    }
-                    // The lane's row goes to the warp's staging tile, 16 bytes at a time, at
-                    // positions swizzled by the row so that neither these stores nor the loads
-                    // of `store_rows` meet in a bank.
-                    const int part = chunk % 2;
-                    if constexpr (SWIGLU) {
-                        // Eight columns hold the gates of four features, then their up
-                        // projections: four outputs, 8 bytes.
-                        #pragma unroll
-                        for (int group = 0; group < CHUNK / 8; group += 2) {
-                            const int slot = part * 2 + group / 2;
-                            *reinterpret_cast<uint4 *>(staging + lane * STAGING_ROW +
-                                                       ((slot ^ (lane & 7)) << 4)) =
-                                make_uint4(
-                                    gated_pair(output, words[group * 4], words[group * 4 + 2]),
-                                    gated_pair(output, words[group * 4 + 1], words[group * 4 + 3]),
-                                    gated_pair(output, words[group * 4 + 4], words[group * 4 + 6]),
-                                    gated_pair(output, words[group * 4 + 5], words[group * 4 + 7]));
-                        }
-                    } else {
-                        #pragma unroll
-                        for (int group = 0; group < CHUNK / 8; group++) {
-                            const int slot = part * 4 + group;
-                            *reinterpret_cast<uint4 *>(staging + lane * STAGING_ROW +
-                                                       ((slot ^ (lane & 7)) << 4)) =
-                                make_uint4(words[group * 4], words[group * 4 + 1],
-                                           words[group * 4 + 2], words[group * 4 + 3]);
-                        }
-                    }
-                };
-                // The 64 staged columns back out by rows: a store instruction covers whole
-                // 128-byte runs of four rows (64-byte runs of eight with SwiGLU) instead of 16
-                // bytes of 32 rows.
-                auto store_rows = [&](int chunk) {
-                    constexpr int SLOTS = SWIGLU ? 4 : 8; // 16-byte pieces of a staged row
-                    constexpr int ROWS_AT_ONCE = 32 / SLOTS;
-                    const int column = first_column + chunk * CHUNK;
-                    const int slot = lane % SLOTS;
-                    __syncwarp();
-                    #pragma unroll
-                    for (int pass = 0; pass < 32 / ROWS_AT_ONCE; pass++) {
-                        const int staged_row = pass * ROWS_AT_ONCE + lane / SLOTS;
-                        const uint4 piece = *reinterpret_cast<const uint4 *>(
-                            staging + staged_row * STAGING_ROW + ((slot ^ (staged_row & 7)) << 4));
-                        if (first_row + staged_row < m) {
-                            Output *destination =
-                                output +
-                                static_cast<size_t>(first_row + staged_row) * output_stride +
-                                (SWIGLU ? column / 2 : column) + slot * 8;
-                            *reinterpret_cast<uint4 *>(destination) = piece;
-                        }
-                    }
-                    __syncwarp();
-                };
-
-                if constexpr (ADAPTED) {
-                    // The product and the adapter's sum of the same 32 columns, side by side.
-                    #pragma unroll
-                    for (int chunk = 0; chunk < TILE_N / 2 / CHUNK; chunk++) {
-                        tmem_load_32(accumulator(0, chunk), even);
-                        tmem_load_32(accumulator(0, chunk) + TMEM_ADAPTER, odd);
-                        tmem_wait_load();
-                        if (chunk == TILE_N / 2 / CHUNK - 1) {
-                            tcgen05_fence_before();
-                            __syncwarp();
-                            if (lane == 0) {
-                                mbar_arrive(barrier(ACCUMULATOR_EMPTY));
-                            }
-                        }
-                        if (!idle) {
-                            scale(even, odd, chunk);
-                            if (chunk % 2 == 1) {
-                                store_rows(chunk - 1);
-                            }
-                        }
-                    }
-                } else {
-                    tmem_wait_load();
-                    tmem_load_32(accumulator(half, 1), odd);
-                    if (!idle) {
-                        scale(even, even, 0);
-                    }
-                    tmem_wait_load();
-                    tmem_load_32(accumulator(half, 2), even);
-                    if (!idle) {
-                        scale(odd, odd, 1);
-                        store_rows(0);
-                    }
-                    tmem_wait_load();
-                    tmem_load_32(accumulator(half, 3), odd);
-                    if (!idle) {
-                        scale(even, even, 2);
-                    }
-                    tmem_wait_load();
-                    if (half + 1 < ROW_TILES) {
-                        tmem_load_32(accumulator(half + 1, 0), even);
-                    } else {
-                        // Everything is out of tensor memory: the next tile's MMAs may start while
-                        // the last columns are scaled and stored.
-                        tcgen05_fence_before();
-                        __syncwarp();
-                        if (lane == 0) {
-                            mbar_arrive(barrier(ACCUMULATOR_EMPTY));
-                        }
-                    }
-                    if (!idle) {
-                        scale(odd, odd, 3);
-                        store_rows(2);
+                        magnitudes = __vmaxu2(magnitudes, words[pair] & 0x7fff7fffu);
                     }
                 }
-                if (track) {
-                    const unsigned magnitude = __reduce_max_sync(
-                        0xffffffffu, max(magnitudes & 0xffffu, magnitudes >> 16));
-                    if (lane == 0 && magnitude != 0) {
-                        // As the FP32 bits of the BF16 magnitude.
-                        atomicMax(maxima + (first_column - maxima_first_column) / 128,
-                                  magnitude << 16);
+                // The lane's row goes to the warp's staging tile, 16 bytes at a time, at
+                // positions swizzled by the row so that neither these stores nor the loads
+                // of `store_rows` meet in a bank.
+                const int part = chunk % 2;
+                if constexpr (SWIGLU) {
+                    // Eight columns hold the gates of four features, then their up
+                    // projections: four outputs, 8 bytes.
+                    #pragma unroll
+                    for (int group = 0; group < CHUNK / 8; group += 2) {
+                        const int slot = part * 2 + group / 2;
+                        *reinterpret_cast<uint4 *>(staging + lane * STAGING_ROW +
+                                                   ((slot ^ (lane & 7)) << 4)) =
+                            make_uint4(
+                                gated_pair(output, words[group * 4], words[group * 4 + 2]),
+                                gated_pair(output, words[group * 4 + 1], words[group * 4 + 3]),
+                                gated_pair(output, words[group * 4 + 4], words[group * 4 + 6]),
+                                gated_pair(output, words[group * 4 + 5], words[group * 4 + 7]));
                     }
+                } else {
+                    #pragma unroll
+                    for (int group = 0; group < CHUNK / 8; group++) {
+                        const int slot = part * 4 + group;
+                        *reinterpret_cast<uint4 *>(staging + lane * STAGING_ROW +
+                                                   ((slot ^ (lane & 7)) << 4)) =
+                            make_uint4(words[group * 4], words[group * 4 + 1],
+                                       words[group * 4 + 2], words[group * 4 + 3]);
+                    }
+                }
+            };
+            // The 64 staged columns back out by rows: a store instruction covers whole
+            // 128-byte runs of four rows (64-byte runs of eight with SwiGLU) instead of 16
+            // bytes of 32 rows.
+            auto store_rows = [&](int chunk) {
+                constexpr int SLOTS = SWIGLU ? 4 : 8; // 16-byte pieces of a staged row
+                constexpr int ROWS_AT_ONCE = 32 / SLOTS;
+                const int column = first_column + chunk * CHUNK;
+                const int slot = lane % SLOTS;
+                __syncwarp();
+                #pragma unroll
+                for (int pass = 0; pass < 32 / ROWS_AT_ONCE; pass++) {
+                    const int staged_row = pass * ROWS_AT_ONCE + lane / SLOTS;
+                    const uint4 piece = *reinterpret_cast<const uint4 *>(
+                        staging + staged_row * STAGING_ROW + ((slot ^ (staged_row & 7)) << 4));
+                    if (first_row + staged_row < m) {
+                        Output *destination =
+                            output +
+                            static_cast<size_t>(first_row + staged_row) * output_stride +
+                            (SWIGLU ? column / 2 : column) + slot * 8;
+                        *reinterpret_cast<uint4 *>(destination) = piece;
+                    }
+                }
+                __syncwarp();
+            };
+
+            if constexpr (ADAPTED) {
+                // The product and the adapter's sum of the same 32 columns, side by side.
+                #pragma unroll
+                for (int chunk = 0; chunk < TILE_N / 2 / CHUNK; chunk++) {
+                    tmem_load_32(accumulator(chunk), even);
+                    tmem_load_32(accumulator(chunk) + TMEM_ADAPTER, odd);
+                    tmem_wait_load();
+                    if (chunk == TILE_N / 2 / CHUNK - 1) {
+                        release();
+                    }
+                    if (!idle) {
+                        scale(even, odd, chunk);
+                        if (chunk % 2 == 1) {
+                            store_rows(chunk - 1);
+                        }
+                    }
+                }
+            } else {
+                tmem_wait_load();
+                tmem_load_32(accumulator(1), odd);
+                if (!idle) {
+                    scale(even, even, 0);
+                }
+                tmem_wait_load();
+                tmem_load_32(accumulator(2), even);
+                if (!idle) {
+                    scale(odd, odd, 1);
+                    store_rows(0);
+                }
+                tmem_wait_load();
+                tmem_load_32(accumulator(3), odd);
+                if (!idle) {
+                    scale(even, even, 2);
+                }
+                tmem_wait_load();
+                // Everything is out of tensor memory: its next tile's MMAs may start while
+                // the last columns are scaled and stored.
+                release();
+                if (!idle) {
+                    scale(odd, odd, 3);
+                    store_rows(2);
+                }
+            }
+            if (track) {
+                const unsigned magnitude = __reduce_max_sync(
+                    0xffffffffu, max(magnitudes & 0xffffu, magnitudes >> 16));
+                if (lane == 0 && magnitude != 0) {
+                    // As the FP32 bits of the BF16 magnitude.
+                    atomicMax(maxima + (first_column - maxima_first_column) / 128,
+                              magnitude << 16);
                 }
             }
         }
@@ -503,17 +511,51 @@ __global__ void __launch_bounds__(THREADS, 1)
 
     tcgen05_fence_before();
     __syncthreads();
-    if (warp == MMA_WARP) {
-        if (*abort_flag != 0) {
-            // A wait gave up: let copies and MMAs in flight land before tensor memory goes back.
-            for (int spin = 0; spin < 64; spin++) {
-                __nanosleep(1000);
-            }
+    if (*abort_flag != 0) {
+        // A wait gave up: let copies and MMAs in flight land before tensor memory goes back.
+        for (int spin = 0; spin < 64; spin++) {
+            __nanosleep(1000);
         }
+    }
+    __syncwarp();
+    // Neither CTA leaves while the other may still reach into it.
+    cluster_sync();
+    if (warp == MMA_WARP) {
         tcgen05_fence_after();
-        tmem_dealloc(tmem, TMEM_COLUMNS);
+        tmem_dealloc_pair(tmem, TMEM_COLUMNS);
     }
 }
+
+// How many pairs of CTAs of `kernel` the device holds at once, asked for once per device.
+struct ResidentPairs {
+    std::atomic<int> counts[MAX_DEVICES];
+    template <typename Kernel> int ask(Kernel kernel) {
+        const int device = current_device();
+        if (device < 0) {
+            return 0;
+        }
+        if (const int kept = counts[device].load(std::memory_order_relaxed); kept != 0) {
+            return kept;
+        }
+        cudaLaunchAttribute cluster;
+        cluster.id = cudaLaunchAttributeClusterDimension;
+        cluster.val.clusterDim.x = 2;
+        cluster.val.clusterDim.y = 1;
+        cluster.val.clusterDim.z = 1;
+        cudaLaunchConfig_t configuration = {};
+        configuration.gridDim = dim3(2);
+        configuration.blockDim = dim3(THREADS);
+        configuration.dynamicSmemBytes = SMEM_BYTES;
+        configuration.attrs = &cluster;
+        configuration.numAttrs = 1;
+        int pairs = 0;
+        if (cudaOccupancyMaxActiveClusters(&pairs, kernel, &configuration) != cudaSuccess) {
+            return 0;
+        }
+        counts[device].store(pairs, std::memory_order_relaxed);
+        return pairs;
+    }
+};
 
 template <typename Output, bool SWIGLU, bool ADAPTED>
 int launch_kernel(const GemmMaps &maps, const float *activation_scales, const float *weight_scales,
@@ -521,27 +563,26 @@ int launch_kernel(const GemmMaps &maps, const float *activation_scales, const fl
                   int band, unsigned *maxima, int maxima_first_column, int rank,
                   float adapter_scale, cudaStream_t stream) {
     unsigned int *status = status_pointer();
-    const int processors = multiprocessor_count();
-    if (status == nullptr || processors == 0) {
-        return static_cast<int>(cudaErrorInvalidDevice);
-    }
-    constexpr int SMEM_BYTES = Shape<ADAPTED>::SMEM_BYTES;
     static SharedMemoryOptIn shared_memory;
+    static ResidentPairs resident;
     const cudaError_t configured =
         shared_memory.ensure(int8_gemm_kernel<Output, SWIGLU, ADAPTED>, SMEM_BYTES);
     if (configured != cudaSuccess) {
         return static_cast<int>(configured);
     }
-    constexpr int TILE_ROWS = Shape<ADAPTED>::ROW_TILES * TILE_M;
+    const int pairs = resident.ask(int8_gemm_kernel<Output, SWIGLU, ADAPTED>);
+    if (status == nullptr || pairs == 0) {
+        return static_cast<int>(cudaErrorInvalidDevice);
+    }
     TileWalk walk;
-    walk.tiles_m = (m + TILE_ROWS - 1) / TILE_ROWS;
+    walk.tiles_m = (m + PAIR_M - 1) / PAIR_M;
     walk.tiles_n = (n + TILE_N - 1) / TILE_N;
     walk.band = band;
     const int64_t tiles = static_cast<int64_t>(walk.tiles_m) * walk.tiles_n;
     if (tiles > INT32_MAX) {
         return INVALID_VALUE;
     }
-    const int blocks = tiles < processors ? static_cast<int>(tiles) : processors;
+    const int blocks = 2 * (tiles < pairs ? static_cast<int>(tiles) : pairs);
     int8_gemm_kernel<Output, SWIGLU, ADAPTED><<<blocks, THREADS, SMEM_BYTES, stream>>>(
         maps, activation_scales, weight_scales, bias, output, m, n, k / BLOCK_K, output_stride,
         walk, maxima, maxima_first_column, ADAPTED ? rank * 2 / BLOCK_K : 0, adapter_scale,
@@ -603,8 +644,8 @@ int launch_int8_gemm(int config, int group_m, const int8_t *activations, const i
     const uint64_t row_dimensions[2] = {static_cast<uint64_t>(k), static_cast<uint64_t>(m)};
     const uint64_t column_dimensions[2] = {static_cast<uint64_t>(k), static_cast<uint64_t>(n)};
     const uint64_t strides[1] = {static_cast<uint64_t>(k)};
-    const uint32_t row_box[2] = {BLOCK_K, static_cast<uint32_t>((adapted ? 1 : 2) * TILE_M)};
-    const uint32_t column_box[2] = {BLOCK_K, TILE_N};
+    const uint32_t row_box[2] = {BLOCK_K, TILE_M};
+    const uint32_t column_box[2] = {BLOCK_K, TILE_N / 2};
     if (!encode_tensor_map(&maps.activations, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, activations,
                            row_dimensions, strides, row_box) ||
         !encode_tensor_map(&maps.weights, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, weights,
@@ -619,7 +660,7 @@ int launch_int8_gemm(int config, int group_m, const int8_t *activations, const i
         const uint64_t down_strides[1] = {static_cast<uint64_t>(adapter_down_stride) * 2};
         const uint64_t up_strides[1] = {static_cast<uint64_t>(rank) * 2};
         const uint32_t down_box[2] = {BLOCK_K / 2, TILE_M};
-        const uint32_t up_box[2] = {BLOCK_K / 2, TILE_N};
+        const uint32_t up_box[2] = {BLOCK_K / 2, TILE_N / 2};
         if (!encode_tensor_map(&maps.adapter_down, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2,
                                adapter_down, down_dimensions, down_strides, down_box) ||
             !encode_tensor_map(&maps.adapter_up, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, adapter_up,

@@ -240,6 +240,67 @@ __device__ __forceinline__ void tmem_store_8(uint32_t address, const uint32_t (&
 }
 
 // ---------------------------------------------------------------------------------------------
+// Pairs of CTAs (clusters of two) on one MMA. A kernel that uses them uses cta_group::2 throughout.
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t rank;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    return rank;
+}
+
+// The address in the cluster of what `address` is in CTA `rank`.
+__device__ __forceinline__ uint32_t cluster_address(uint32_t address, uint32_t rank) {
+    uint32_t mapped;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(mapped) : "r"(address), "r"(rank));
+    return mapped;
+}
+
+// Every thread of both CTAs. It has no limit of its own: each CTA gets here because every wait
+// before it has one.
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n"
+                 "barrier.cluster.wait.acquire.aligned;" ::
+                     : "memory");
+}
+
+// `bar` is a cluster_address.
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar)
+                 : "memory");
+}
+
+// Into this CTA's shared memory, counted by a barrier of either CTA of the pair (`bar` is a
+// cluster_address).
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t destination, const CUtensorMap *map,
+                                                 uint32_t bar, int c0, int c1) {
+    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+                 ".cta_group::2 [%0], [%1, {%3, %4}], [%2];" ::"r"(destination),
+                 "l"(map), "r"(bar), "r"(c0), "r"(c1)
+                 : "memory");
+}
+
+__device__ __forceinline__ void tmem_alloc_pair(uint32_t destination, uint32_t columns) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     destination),
+                 "r"(columns)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+
+__device__ __forceinline__ void tmem_dealloc_pair(uint32_t base, uint32_t columns) {
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(base), "r"(columns)
+                 : "memory");
+}
+
+// Makes `bar` of both CTAs complete once every pair MMA this thread has issued so far has.
+__device__ __forceinline__ void tcgen05_commit_pair(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster"
+                 ".multicast::cluster.b64 [%0], %1;" ::"r"(bar),
+                 "h"(static_cast<uint16_t>(3))
+                 : "memory");
+}
+
+// ---------------------------------------------------------------------------------------------
 // UMMA descriptors
 
 // Shared-memory matrix descriptor of a tile in the 128-byte swizzle TMA writes (rows of 128 bytes,
@@ -290,13 +351,13 @@ __host__ __device__ constexpr uint32_t instruction_descriptor(uint32_t accumulat
 }
 
 // D (TMEM) = A (smem) · B (smem), or D += A · B when `accumulate` is nonzero. One thread issues it.
-#define MMH3_DEFINE_MMA(KIND, NAME)                                                               \
+#define MMH3_DEFINE_MMA(GROUP, KIND, NAME)                                                        \
     __device__ __forceinline__ void NAME##_ss(uint32_t d, uint64_t a, uint64_t b,                 \
                                               uint32_t instruction, uint32_t accumulate) {        \
         asm volatile("{\n"                                                                        \
                      ".reg .pred p;\n"                                                            \
                      "setp.ne.b32 p, %4, 0;\n"                                                    \
-                     "tcgen05.mma.cta_group::1.kind::" KIND " [%0], %1, %2, %3, p;\n"             \
+                     "tcgen05.mma." GROUP ".kind::" KIND " [%0], %1, %2, %3, p;\n"                \
                      "}" ::"r"(d),                                                                \
                      "l"(a), "l"(b), "r"(instruction), "r"(accumulate)                            \
                      : "memory");                                                                 \
@@ -307,15 +368,19 @@ __host__ __device__ constexpr uint32_t instruction_descriptor(uint32_t accumulat
         asm volatile("{\n"                                                                        \
                      ".reg .pred p;\n"                                                            \
                      "setp.ne.b32 p, %4, 0;\n"                                                    \
-                     "tcgen05.mma.cta_group::1.kind::" KIND " [%0], [%1], %2, %3, p;\n"           \
+                     "tcgen05.mma." GROUP ".kind::" KIND " [%0], [%1], %2, %3, p;\n"              \
                      "}" ::"r"(d),                                                                \
                      "r"(a), "l"(b), "r"(instruction), "r"(accumulate)                            \
                      : "memory");                                                                 \
     }
 
-MMH3_DEFINE_MMA("f16", mma_f16)
-MMH3_DEFINE_MMA("i8", mma_i8)
-MMH3_DEFINE_MMA("f8f6f4", mma_f8)
+MMH3_DEFINE_MMA("cta_group::1", "f16", mma_f16)
+MMH3_DEFINE_MMA("cta_group::1", "i8", mma_i8)
+MMH3_DEFINE_MMA("cta_group::1", "f8f6f4", mma_f8)
+// The same over a pair of CTAs, issued by one thread of the pair's first: M = 256, each CTA with
+// 128 rows of A and of D and half of B's rows, at the same places of its own memories.
+MMH3_DEFINE_MMA("cta_group::2", "f16", mma_f16_pair)
+MMH3_DEFINE_MMA("cta_group::2", "i8", mma_i8_pair)
 #undef MMH3_DEFINE_MMA
 
 // Moves registers between the warpgroups of a CTA: every warp of a warpgroup (four consecutive

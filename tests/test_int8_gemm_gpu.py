@@ -109,6 +109,38 @@ def test_matches_the_definition_oracle_and_reference(oracle, reference_kernels, 
             assert np.array_equal(maxima, other_maxima)
 
 
+@pytest.mark.parametrize("m,n,k", [
+    (1, 128, 128),       # one row, a tile of 128 columns, one stage
+    (128, 256, 768),     # the second CTA of a pair without rows; as many stages as the ring has
+    (129, 384, 896),     # one row for it; one stage more
+    (520, 13184, 128),   # more tiles than pairs of CTAs: an accumulator's second and third tile
+    (513, 13312, 1024),
+    (2305, 7936, 256),
+])
+def test_tiles_of_cta_pairs(oracle, m, n, k):
+    """Two CTAs share a tile of 256 rows and take turns with two accumulators."""
+    case = gemm_cases.operands(m, n, k, m + k)
+    bits, maxima = run(case, m, n, k, first_column=0)
+    expected, expected_maxima = oracle_lib.int8_gemm(oracle, *case, maxima_first_column=0)
+    assert np.array_equal(bits, expected)
+    assert np.array_equal(maxima, expected_maxima)
+
+
+@pytest.mark.parametrize("m,n,k,rank", [
+    (1, 128, 128, 64), (129, 384, 640, 128), (513, 13312, 256, 64), (300, 28672, 384, 384),
+])
+def test_tiles_of_cta_pairs_with_an_adapter(m, n, k, rank):
+    # The bounds of test_adds_a_low_rank_adapter.
+    case = gemm_cases.operands(m, n, k, m + k)
+    down, up = gemm_cases.adapter_operands(m, n, rank, rank, 7)
+    adapter = (down, up, rank, 1.5)
+    bits, maxima = run(case, m, n, k, first_column=0, adapter=adapter)
+    expected = gemm_cases.definition(*case, adapter=adapter)
+    actual = gemm_cases.widen(bits, False)
+    assert np.all(np.abs(actual - expected) <= np.abs(expected) / 256.0 + 1e-4)
+    assert np.array_equal(maxima, gemm_cases.column_maxima(bits, 0))
+
+
 @pytest.mark.parametrize("f16", [False, True])
 def test_swiglu_of_interleaved_rows(oracle, reference_kernels, f16):
     # int8_gemm.rs:269-383 without the adapter; the rows interleaved by the library itself.
