@@ -353,73 +353,110 @@ __global__ void __launch_bounds__(THREADS, 1)
         bool alive = true;
         if constexpr (ROPE) {
             // The eight softmax warps normalize and rotate the 256 query rows where TMA left them,
-            // a warp to a row: lane l holds dimensions l, l + 32, ... of the row.
+            // a warp to a row. A lane takes both dimensions of its pairs, so that nothing crosses
+            // lanes but the sum of squares and a pair's sine and cosine are computed once, and then
+            // its share of the dimensions behind the pairs. A row alone is a chain of loads,
+            // shuffles and sincosf, so a warp has ROWS_AT_ONCE of them under way: eight windows of
+            // 1,025 tokens with 16 heads of 64 and 32 pairs took 180 us with a row at a time and
+            // every sine and cosine computed twice, and take 138.
             alive = mbar_wait(barrier(QUERY_FULL), 0, watchdog, STATUS_DENSE | 10);
             alive = __all_sync(0xffffffffu, alive);
-            constexpr int SLOTS = DIM / 32;
-            for (int query_row = warp; alive && query_row < QUERY_TILES * TILE_M;
-                 query_row += SOFTMAX_WARPS) {
-                const int token = first_query + query_row;
-                if (token >= tokens) {
-                    continue;
-                }
+            constexpr int PAIR_SLOTS = DIM / 64;  // pairs of a lane: 2 * pairs <= DIM
+            constexpr int OTHER_SLOTS = DIM / 32; // dimensions behind the pairs
+            constexpr int ROWS_AT_ONCE = 4;
+            constexpr int ROWS_OF_WARP = QUERY_TILES * TILE_M / SOFTMAX_WARPS;
+            static_assert(ROWS_OF_WARP % ROWS_AT_ONCE == 0, "no rows are left over");
+            const int others = DIM - 2 * rope.pairs;
+            // Where dimension `index` of query row `query_row` lies: 16-byte chunk c of a row sits
+            // at chunk c ^ (row % 8) of its 128-byte line.
+            auto address = [&](int query_row, int index) {
                 const int tile_row = query_row % TILE_M;
-                uint32_t addresses[SLOTS];
-                float values[SLOTS];
-                float squares = 0.0f;
+                const int chunk = ((index % 64) / 8) ^ (tile_row % 8);
+                return base + SMEM_QUERY + (query_row / TILE_M) * TILE_BYTES +
+                       (index / 64) * SLAB_BYTES + tile_row * 128 + chunk * 16 + (index % 8) * 2;
+            };
+            auto load = [&](int query_row, int index) {
+                uint16_t bits;
+                asm volatile("ld.shared.u16 %0, [%1];" : "=h"(bits) : "r"(address(query_row, index)));
+                return Element<HALF, DIM>::to_float(bits);
+            };
+            auto store = [&](int query_row, int index, float value) {
+                const uint16_t bits = Element<HALF, DIM>::from_float(value);
+                asm volatile("st.shared.u16 [%0], %1;" ::"r"(address(query_row, index)), "h"(bits)
+                             : "memory");
+            };
+            const int rows_here = alive ? min(tokens - first_query, QUERY_TILES * TILE_M) : 0;
+            const int warp_end = min(rows_here, (warp + 1) * ROWS_OF_WARP);
+            #pragma unroll 1
+            for (int first_row = warp * ROWS_OF_WARP; first_row < warp_end;
+                 first_row += ROWS_AT_ONCE) {
+                // Rows past the last token are zeroes; they are worked on and stored like the rest,
+                // with the last token's angles.
+                float angle[ROWS_AT_ONCE][PAIR_SLOTS];
+                float first[ROWS_AT_ONCE][PAIR_SLOTS], second[ROWS_AT_ONCE][PAIR_SLOTS];
+                float other[ROWS_AT_ONCE][OTHER_SLOTS];
+                float squares[ROWS_AT_ONCE];
                 #pragma unroll
-                for (int slot = 0; slot < SLOTS; slot++) {
-                    const int index = slot * 32 + lane;
-                    // 16-byte chunk c of a row sits at chunk c ^ (row % 8) of its 128-byte line.
-                    const int chunk = ((index % 64) / 8) ^ (tile_row % 8);
-                    addresses[slot] = base + SMEM_QUERY + (query_row / TILE_M) * TILE_BYTES +
-                                      (index / 64) * SLAB_BYTES + tile_row * 128 + chunk * 16 +
-                                      (index % 8) * 2;
-                    uint16_t bits;
-                    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(bits) : "r"(addresses[slot]));
-                    values[slot] = Element<HALF, DIM>::to_float(bits);
-                    squares = fmaf(values[slot], values[slot], squares);
+                for (int at = 0; at < ROWS_AT_ONCE; at++) {
+                    const int token = min(first_query + first_row + at, tokens - 1);
+                    #pragma unroll
+                    for (int slot = 0; slot < PAIR_SLOTS; slot++) {
+                        const int pair = slot * 32 + lane;
+                        angle[at][slot] =
+                            pair < rope.pairs
+                                ? __ldg(rope.angles + static_cast<int64_t>(token) * rope.pairs + pair)
+                                : 0.0f;
+                    }
+                }
+                #pragma unroll
+                for (int at = 0; at < ROWS_AT_ONCE; at++) {
+                    squares[at] = 0.0f;
+                    #pragma unroll
+                    for (int slot = 0; slot < PAIR_SLOTS; slot++) {
+                        const int pair = slot * 32 + lane;
+                        const bool here = pair < rope.pairs;
+                        first[at][slot] = here ? load(first_row + at, pair) : 0.0f;
+                        second[at][slot] = here ? load(first_row + at, pair + rope.pairs) : 0.0f;
+                        squares[at] = fmaf(first[at][slot], first[at][slot], squares[at]);
+                        squares[at] = fmaf(second[at][slot], second[at][slot], squares[at]);
+                    }
+                    #pragma unroll
+                    for (int slot = 0; slot < OTHER_SLOTS; slot++) {
+                        const int index = slot * 32 + lane;
+                        other[at][slot] =
+                            index < others ? load(first_row + at, 2 * rope.pairs + index) : 0.0f;
+                        squares[at] = fmaf(other[at][slot], other[at][slot], squares[at]);
+                    }
                 }
                 #pragma unroll
                 for (int offset = 16; offset > 0; offset /= 2) {
-                    squares += __shfl_xor_sync(0xffffffffu, squares, offset);
-                }
-                const float inverse = rsqrtf(squares / DIM + rope.epsilon);
-                #pragma unroll
-                for (int slot = 0; slot < SLOTS; slot++) {
-                    values[slot] *= inverse;
-                }
-                float rotated[SLOTS];
-                #pragma unroll
-                for (int slot = 0; slot < SLOTS; slot++) {
-                    const int index = slot * 32 + lane;
-                    const bool leads = index < rope.pairs;
-                    const bool follows = !leads && index < 2 * rope.pairs;
-                    const int partner = leads ? index + rope.pairs
-                                              : (follows ? index - rope.pairs : index);
-                    float other = 0.0f;
                     #pragma unroll
-                    for (int source = 0; source < SLOTS; source++) {
-                        const float fetched =
-                            __shfl_sync(0xffffffffu, values[source], partner % 32);
-                        other = source == partner / 32 ? fetched : other;
+                    for (int at = 0; at < ROWS_AT_ONCE; at++) {
+                        squares[at] += __shfl_xor_sync(0xffffffffu, squares[at], offset);
                     }
-                    float result = values[slot];
-                    if (leads || follows) {
-                        float sine, cosine;
-                        sincosf(rope.angles[static_cast<int64_t>(token) * rope.pairs +
-                                            (leads ? index : partner)],
-                                &sine, &cosine);
-                        result = leads ? values[slot] * cosine - other * sine
-                                       : other * sine + values[slot] * cosine;
-                    }
-                    rotated[slot] = result;
                 }
                 #pragma unroll
-                for (int slot = 0; slot < SLOTS; slot++) {
-                    const uint16_t bits = Element<HALF, DIM>::from_float(rotated[slot]);
-                    asm volatile("st.shared.u16 [%0], %1;" ::"r"(addresses[slot]), "h"(bits)
-                                 : "memory");
+                for (int at = 0; at < ROWS_AT_ONCE; at++) {
+                    const float inverse = rsqrtf(squares[at] / DIM + rope.epsilon);
+                    #pragma unroll
+                    for (int slot = 0; slot < PAIR_SLOTS; slot++) {
+                        const int pair = slot * 32 + lane;
+                        if (pair < rope.pairs) {
+                            float sine, cosine;
+                            sincosf(angle[at][slot], &sine, &cosine);
+                            const float one = first[at][slot] * inverse;
+                            const float two = second[at][slot] * inverse;
+                            store(first_row + at, pair, one * cosine - two * sine);
+                            store(first_row + at, pair + rope.pairs, one * sine + two * cosine);
+                        }
+                    }
+                    #pragma unroll
+                    for (int slot = 0; slot < OTHER_SLOTS; slot++) {
+                        const int index = slot * 32 + lane;
+                        if (index < others) {
+                            store(first_row + at, 2 * rope.pairs + index, other[at][slot] * inverse);
+                        }
+                    }
                 }
             }
             // The MMAs read the tiles through the async proxy.

@@ -354,6 +354,35 @@ def test_heads_of_64_and_the_fused_query_rope(reference_kernels, element_type, h
     assert cosine(a, b) >= 0.9995
 
 
+@pytest.mark.parametrize("head_dim,tokens,pairs", [
+    (64, 1, 32), (64, 127, 20), (64, 129, 1), (64, 257, 31), (64, 518, 32),
+    (128, 5, 64), (128, 131, 33), (128, 300, 40), (128, 255, 3),
+])
+@pytest.mark.parametrize("element_type", [0, 1])
+def test_fused_query_rope_against_float64(element_type, head_dim, tokens, pairs):
+    """Every split of a head into pairs and the rest, rows that fill a warp's turn and rows that do
+    not; the bound of the tests above."""
+    heads, batch, epsilon = 3, 2, 1e-6
+    scale = 1.0 / head_dim ** 0.5
+    dtype = torch.float16 if element_type == 1 else torch.bfloat16
+    generator = torch.Generator().manual_seed(tokens + head_dim + pairs)
+    q, k, v = (torch.randn((batch, tokens, heads, head_dim), generator=generator).to(dtype)
+               for _ in range(3))
+    q = q * 3
+    inner = heads * head_dim
+    layout = attention.make_layout((inner,) * 4, head_stride=(head_dim,) * 4,
+                                   batch_stride=(tokens * inner,) * 4)
+    angles = torch.rand((tokens, pairs), generator=generator) * 80.0 - 40.0
+    ours = torch.zeros((batch, tokens, heads, head_dim), dtype=dtype, device="cuda")
+    attention.attention_roped(element_type, head_dim, q.cuda(), k.cuda(), v.cuda(), ours, tokens,
+                              heads, batch, layout, scale, angles.cuda(), pairs, epsilon)
+    assert attention.take_status() == 0
+    query = normalized_rotated(q, angles, pairs, epsilon, dtype)
+    scores = torch.einsum("bqhd,bkhd->bhqk", query.double(), k.double()) * scale
+    expected = torch.einsum("bhqk,bkhd->bqhd", scores.softmax(-1), v.double())
+    assert torch.max(torch.abs(ours.cpu().double() - expected)) <= 2e-2
+
+
 def test_unsupported_combinations_report_an_error():
     tokens, heads = 64, 1
     qkv = torch.zeros((tokens, 3, heads, 128), dtype=torch.bfloat16, device="cuda")
