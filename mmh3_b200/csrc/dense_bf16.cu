@@ -68,8 +68,8 @@ template <int DIM> struct Shape {
 };
 
 enum Barrier {
-    QUERY_FULL = 0,
-    RING_FULL = 1,
+    QUERY_FULL = 0,                                  // one per query tile
+    RING_FULL = QUERY_FULL + QUERY_TILES,
     RING_EMPTY = RING_FULL + STAGES,
     SCORES_FULL = RING_EMPTY + STAGES,               // one per query tile
     PROBABILITIES_FULL = SCORES_FULL + QUERY_TILES,  // one per query tile
@@ -195,12 +195,12 @@ __global__ void __launch_bounds__(THREADS, 1)
                               : (tokens + TILE_N - 1) / TILE_N;
 
     if (threadIdx.x == 0) {
-        mbar_init(barrier(QUERY_FULL), 1);
         for (int stage = 0; stage < STAGES; stage++) {
             mbar_init(barrier(RING_FULL + stage), 1);
             mbar_init(barrier(RING_EMPTY + stage), 1);
         }
         for (int tile = 0; tile < QUERY_TILES; tile++) {
+            mbar_init(barrier(QUERY_FULL + tile), 1);
             mbar_init(barrier(SCORES_FULL + tile), 1);
             mbar_init(barrier(PROBABILITIES_FULL + tile), TILE_M);
             mbar_init(barrier(PROBABILITIES_HALF + tile), TILE_M);
@@ -228,14 +228,15 @@ __global__ void __launch_bounds__(THREADS, 1)
             tma_prefetch_descriptor(&maps.key);
             tma_prefetch_descriptor(&maps.value);
             const int key_value_head = head / heads_per_key_value;
-            mbar_expect_tx(barrier(QUERY_FULL), QUERY_TILES * TILE_BYTES);
-            for (int tile = 0; tile < QUERY_TILES; tile++) {
+            auto load_query = [&](int tile) {
+                mbar_expect_tx(barrier(QUERY_FULL + tile), TILE_BYTES);
                 for (int slab = 0; slab < SLABS; slab++) {
                     tma_load_4d(base + SMEM_QUERY + tile * TILE_BYTES + slab * SLAB_BYTES,
-                                &maps.query, barrier(QUERY_FULL), slab * 64,
+                                &maps.query, barrier(QUERY_FULL + tile), slab * 64,
                                 first_query + tile * TILE_M, head, item_of_batch);
                 }
-            }
+            };
+            load_query(0);
             // K0, V0, K1, V1, ... in the order the MMA warp consumes and releases them.
             for (int item = 0; item < 2 * blocks; item++) {
                 const int stage = item % STAGES;
@@ -250,6 +251,10 @@ __global__ void __launch_bounds__(THREADS, 1)
                     tma_load_4d(base + SMEM_RING + stage * TILE_BYTES + slab * SLAB_BYTES, map,
                                 barrier(RING_FULL + stage), slab * 64, (item / 2) * TILE_N,
                                 key_value_head, item_of_batch);
+                }
+                if (item == 0) {
+                    // Behind what the first scores need.
+                    load_query(1);
                 }
             }
         }
@@ -287,6 +292,10 @@ __global__ void __launch_bounds__(THREADS, 1)
             if (alive) {
                 tcgen05_fence_after();
                 score(0, ring);
+                alive = ROPE || mbar_wait(barrier(QUERY_FULL + 1), 0, watchdog, STATUS_DENSE | 2);
+            }
+            if (alive) {
+                tcgen05_fence_after();
                 score(1, ring);
                 tcgen05_commit(barrier(RING_EMPTY + 0));
             }
@@ -359,7 +368,7 @@ __global__ void __launch_bounds__(THREADS, 1)
             // shuffles and sincosf, so a warp has ROWS_AT_ONCE of them under way: eight windows of
             // 1,025 tokens with 16 heads of 64 and 32 pairs took 180 us with a row at a time and
             // every sine and cosine computed twice, and take 138.
-            alive = mbar_wait(barrier(QUERY_FULL), 0, watchdog, STATUS_DENSE | 10);
+            alive = mbar_wait(barrier(QUERY_FULL + warp / 4), 0, watchdog, STATUS_DENSE | 10);
             alive = __all_sync(0xffffffffu, alive);
             constexpr int PAIR_SLOTS = DIM / 64;  // pairs of a lane: 2 * pairs <= DIM
             constexpr int OTHER_SLOTS = DIM / 32; // dimensions behind the pairs
@@ -574,37 +583,43 @@ __global__ void __launch_bounds__(THREADS, 1)
             uint16_t *output_row = output + static_cast<int64_t>(token) * output_token_stride +
                                    static_cast<int64_t>(head) * output_head_stride +
                                    item_of_batch * output_batch_stride;
+            // The query tiles are at rest: the warp's rows leave through 32 of theirs. Stored from
+            // where they are, a lane's row 16 bytes at a time, they held up a CTA for 6,000 to
+            // 8,000 cycles, as long as two blocks of keys (a BF16 attention layer of 1,101 tokens
+            // and 56 heads: 191 us, 187 this way).
+            const StagedRows<DIM> staged{base + SMEM_QUERY + warp * (32 * DIM * 2)};
             #pragma unroll
             for (int chunk = 0; chunk < DIM / 32; chunk++) {
                 uint32_t values[32];
                 tmem_load_32(accumulator + chunk * 32, values);
                 tmem_wait_load();
-                if (token < tokens) {
-                    uint32_t packed[16];
+                uint32_t packed[16];
+                #pragma unroll
+                for (int pair = 0; pair < 16; pair++) {
+                    packed[pair] =
+                        Element<HALF, DIM>::pack(__uint_as_float(values[pair * 2]) * inverse,
+                                                 __uint_as_float(values[pair * 2 + 1]) * inverse);
+                }
+                if (vector_stores) {
+                    #pragma unroll
+                    for (int part = 0; part < 4; part++) {
+                        staged.put(lane, chunk * 4 + part,
+                                   make_uint4(packed[part * 4], packed[part * 4 + 1],
+                                              packed[part * 4 + 2], packed[part * 4 + 3]));
+                    }
+                } else if (token < tokens) {
+                    uint16_t *destination = output_row + chunk * 32;
                     #pragma unroll
                     for (int pair = 0; pair < 16; pair++) {
-                        packed[pair] =
-                            Element<HALF, DIM>::pack(__uint_as_float(values[pair * 2]) * inverse,
-                                                __uint_as_float(values[pair * 2 + 1]) * inverse);
-                    }
-                    if (vector_stores) {
-                        uint4 *destination = reinterpret_cast<uint4 *>(output_row + chunk * 32);
-                        #pragma unroll
-                        for (int part = 0; part < 4; part++) {
-                            destination[part] =
-                                make_uint4(packed[part * 4], packed[part * 4 + 1],
-                                           packed[part * 4 + 2], packed[part * 4 + 3]);
-                        }
-                    } else {
-                        uint16_t *destination =
-                            reinterpret_cast<uint16_t *>(output_row + chunk * 32);
-                        #pragma unroll
-                        for (int pair = 0; pair < 16; pair++) {
-                            destination[pair * 2] = static_cast<uint16_t>(packed[pair] & 0xffffu);
-                            destination[pair * 2 + 1] = static_cast<uint16_t>(packed[pair] >> 16);
-                        }
+                        destination[pair * 2] = static_cast<uint16_t>(packed[pair] & 0xffffu);
+                        destination[pair * 2 + 1] = static_cast<uint16_t>(packed[pair] >> 16);
                     }
                 }
+            }
+            if (vector_stores) {
+                // From the warp's first row on.
+                staged.store(output_row - lane * output_token_stride, output_token_stride,
+                             tokens - (token - lane));
             }
         }
     }

@@ -56,8 +56,8 @@ constexpr int SMEM_BARRIERS = SMEM_RING + STAGES * TILE_BYTES;
 constexpr int SMEM_BYTES = SMEM_BARRIERS + 256 + 1024;
 
 enum Barrier {
-    QUERY_FULL = 0,
-    RING_FULL = 1,
+    QUERY_FULL = 0, // one per query tile
+    RING_FULL = QUERY_FULL + QUERY_TILES,
     RING_EMPTY = RING_FULL + STAGES,
     SCORES_FULL = RING_EMPTY + STAGES,
     PROBABILITIES_FULL = SCORES_FULL + QUERY_TILES,
@@ -129,12 +129,12 @@ __global__ void __launch_bounds__(THREADS, 1)
     const int blocks = (tokens + TILE_N - 1) / TILE_N;
 
     if (threadIdx.x == 0) {
-        mbar_init(barrier(QUERY_FULL), 1);
         for (int stage = 0; stage < STAGES; stage++) {
             mbar_init(barrier(RING_FULL + stage), 1);
             mbar_init(barrier(RING_EMPTY + stage), 1);
         }
         for (int tile = 0; tile < QUERY_TILES; tile++) {
+            mbar_init(barrier(QUERY_FULL + tile), 1);
             mbar_init(barrier(SCORES_FULL + tile), 1);
             mbar_init(barrier(PROBABILITIES_FULL + tile), TILE_M);
         }
@@ -159,11 +159,12 @@ __global__ void __launch_bounds__(THREADS, 1)
             tma_prefetch_descriptor(&maps.query);
             tma_prefetch_descriptor(&maps.key);
             tma_prefetch_descriptor(&maps.value);
-            mbar_expect_tx(barrier(QUERY_FULL), QUERY_TILES * TILE_BYTES);
-            for (int tile = 0; tile < QUERY_TILES; tile++) {
+            auto load_query = [&](int tile) {
+                mbar_expect_tx(barrier(QUERY_FULL + tile), TILE_BYTES);
                 tma_load_3d(base + SMEM_QUERY + tile * TILE_BYTES, &maps.query,
-                            barrier(QUERY_FULL), 0, first_query + tile * TILE_M, head);
-            }
+                            barrier(QUERY_FULL + tile), 0, first_query + tile * TILE_M, head);
+            };
+            load_query(0);
             for (int item = 0; item < 2 * blocks; item++) {
                 const int stage = item % STAGES;
                 const int use = item / STAGES;
@@ -180,6 +181,10 @@ __global__ void __launch_bounds__(THREADS, 1)
                 } else {
                     tma_load_3d(destination, &maps.key, barrier(RING_FULL + stage), 0,
                                 (item / 2) * TILE_N, head);
+                }
+                if (item == 0) {
+                    // Behind what the first scores need.
+                    load_query(1);
                 }
             }
         }
@@ -215,6 +220,10 @@ __global__ void __launch_bounds__(THREADS, 1)
             if (alive) {
                 tcgen05_fence_after();
                 score(0, ring);
+                alive = mbar_wait(barrier(QUERY_FULL + 1), 0, watchdog, STATUS_QUANTIZED | 2);
+            }
+            if (alive) {
+                tcgen05_fence_after();
                 score(1, ring);
                 tcgen05_commit(barrier(RING_EMPTY + 0));
             }
@@ -418,36 +427,44 @@ __global__ void __launch_bounds__(THREADS, 1)
             __nv_bfloat16 *output_row =
                 output + static_cast<int64_t>(token) * output_token_stride +
                 static_cast<int64_t>(head) * output_head_stride;
+            // The query tiles and the ring are at rest: the warp's rows leave through 8 KB of them.
+            // Stored from where they are, a lane's row 16 bytes at a time, they took 7,500 cycles
+            // of a CTA, as much as two blocks of keys (2,085 tokens and 56 heads with their
+            // quantization: 221 us, 213 this way).
+            const StagedRows<HEAD_DIM> staged{base + SMEM_QUERY + warp * (32 * HEAD_DIM * 2)};
+            static_assert(SOFTMAX_WARPS * 32 * HEAD_DIM * 2 <= SMEM_BARRIERS,
+                          "the staged rows fit before the barriers");
             #pragma unroll
             for (int chunk = 0; chunk < 4; chunk++) {
                 uint32_t values[32];
                 tmem_load_32(accumulator + chunk * 32, values);
                 tmem_wait_load();
-                if (token < tokens) {
-                    uint32_t packed[16];
+                uint32_t packed[16];
+                #pragma unroll
+                for (int pair = 0; pair < 16; pair++) {
+                    packed[pair] = pack_bf16(__uint_as_float(values[pair * 2]) * inverse,
+                                             __uint_as_float(values[pair * 2 + 1]) * inverse);
+                }
+                if (vector_stores) {
+                    #pragma unroll
+                    for (int part = 0; part < 4; part++) {
+                        staged.put(lane, chunk * 4 + part,
+                                   make_uint4(packed[part * 4], packed[part * 4 + 1],
+                                              packed[part * 4 + 2], packed[part * 4 + 3]));
+                    }
+                } else if (token < tokens) {
+                    uint16_t *destination = reinterpret_cast<uint16_t *>(output_row + chunk * 32);
                     #pragma unroll
                     for (int pair = 0; pair < 16; pair++) {
-                        packed[pair] = pack_bf16(__uint_as_float(values[pair * 2]) * inverse,
-                                                 __uint_as_float(values[pair * 2 + 1]) * inverse);
-                    }
-                    if (vector_stores) {
-                        uint4 *destination = reinterpret_cast<uint4 *>(output_row + chunk * 32);
-                        #pragma unroll
-                        for (int part = 0; part < 4; part++) {
-                            destination[part] =
-                                make_uint4(packed[part * 4], packed[part * 4 + 1],
-                                           packed[part * 4 + 2], packed[part * 4 + 3]);
-                        }
-                    } else {
-                        uint16_t *destination =
-                            reinterpret_cast<uint16_t *>(output_row + chunk * 32);
-                        #pragma unroll
-                        for (int pair = 0; pair < 16; pair++) {
-                            destination[pair * 2] = static_cast<uint16_t>(packed[pair] & 0xffffu);
-                            destination[pair * 2 + 1] = static_cast<uint16_t>(packed[pair] >> 16);
-                        }
+                        destination[pair * 2] = static_cast<uint16_t>(packed[pair] & 0xffffu);
+                        destination[pair * 2 + 1] = static_cast<uint16_t>(packed[pair] >> 16);
                     }
                 }
+            }
+            if (vector_stores) {
+                // From the warp's first row on.
+                staged.store(reinterpret_cast<uint16_t *>(output_row - lane * output_token_stride),
+                             output_token_stride, tokens - (token - lane));
             }
         }
     }

@@ -393,6 +393,43 @@ template <int REGISTERS> __device__ __forceinline__ void register_decrease() {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGISTERS));
 }
 
+// 32 rows of DIM 16-bit values on their way from a warp that holds a row per lane to global memory,
+// through a corner of shared memory of the warp's own (32 * DIM * 2 bytes, on 16 bytes), so that a
+// store covers whole rows instead of 16 bytes of each of 32. Piece c (16 bytes) of row r lies at
+// piece c ^ (r % 8): neither the rows' pieces going in nor the rows coming out meet in a bank.
+template <int DIM> struct StagedRows {
+    static constexpr int PIECES = DIM / 8;
+    static constexpr int ROWS_AT_ONCE = 32 / PIECES;
+    uint32_t rows_base; // shared-memory address
+
+    __device__ __forceinline__ uint32_t address(int row, int piece) const {
+        return rows_base + (row * PIECES + (piece ^ (row % 8))) * 16;
+    }
+    __device__ __forceinline__ void put(int row, int piece, uint4 value) const {
+        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(address(row, piece)),
+                     "r"(value.x), "r"(value.y), "r"(value.z), "r"(value.w)
+                     : "memory");
+    }
+    // The first `rows` rows, `stride` elements apart. The whole warp calls it.
+    __device__ __forceinline__ void store(uint16_t *output, int64_t stride, int rows) const {
+        const int lane = threadIdx.x % 32;
+        const int piece = lane % PIECES;
+        __syncwarp();
+        #pragma unroll
+        for (int pass = 0; pass < 32 / ROWS_AT_ONCE; pass++) {
+            const int row = pass * ROWS_AT_ONCE + lane / PIECES;
+            if (row < rows) {
+                uint4 value;
+                asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+                             : "=r"(value.x), "=r"(value.y), "=r"(value.z), "=r"(value.w)
+                             : "r"(address(row, piece))
+                             : "memory");
+                *reinterpret_cast<uint4 *>(output + row * stride + piece * 8) = value;
+            }
+        }
+    }
+};
+
 __device__ __forceinline__ float exp2_approx(float value) {
     float result;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(result) : "f"(value));
