@@ -179,10 +179,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     const Watchdog watchdog = {abort_flag, status};
     auto barrier = [&](int index) { return barriers + index * 8; };
 
-    // Once a wait has run out anywhere, the rest of the grid drains instead of waiting too.
-    if (*reinterpret_cast<volatile unsigned int *>(status) != 0) {
-        return;
-    }
+    let_next_kernel_begin();
     const int warp = warp_index();
     const int lane = threadIdx.x % 32;
     const int head = blockIdx.y;
@@ -214,10 +211,18 @@ __global__ void __launch_bounds__(THREADS, 1)
     if (warp == MMA_WARP) {
         tmem_alloc(smem_u32(const_cast<uint32_t *>(tmem_slot)), TMEM_COLUMNS);
     }
+    wait_for_kernels_before();
     tcgen05_fence_before();
-    __syncthreads();
+    // Once a wait has run out anywhere, the rest of the grid drains instead of waiting too.
+    const bool stopped = __syncthreads_or(*reinterpret_cast<volatile unsigned int *>(status) != 0);
     tcgen05_fence_after();
     const uint32_t tmem = *tmem_slot;
+    if (stopped) {
+        if (warp == MMA_WARP) {
+            tmem_dealloc(tmem, TMEM_COLUMNS);
+        }
+        return;
+    }
 
     if (warp >= SOFTMAX_WARPS) {
         register_decrease<OTHER_REGISTERS>();
@@ -804,11 +809,10 @@ int launch_dense_bf16(const void *query, const void *key, const void *value, voi
                                   layout.head_stride[OUTPUT] % 8 == 0 &&
                                   (items == 1 || layout.batch_stride[OUTPUT] % 8 == 0);
         const dim3 grid((tokens + QUERY_TILES * TILE_M - 1) / (QUERY_TILES * TILE_M), heads, items);
-        chosen.kernel<<<grid, THREADS, chosen.shared_bytes, stream>>>(
-            maps, batch_output, tokens, group, layout.token_stride[OUTPUT],
-            layout.head_stride[OUTPUT], layout.batch_stride[OUTPUT], vector_stores,
-            scale * LOG2_E, query_rope, status);
-        const cudaError_t launched = cudaGetLastError();
+        const cudaError_t launched = launch_behind(
+            chosen.kernel, grid, THREADS, chosen.shared_bytes, stream, maps, batch_output, tokens,
+            group, layout.token_stride[OUTPUT], layout.head_stride[OUTPUT],
+            layout.batch_stride[OUTPUT], vector_stores, scale * LOG2_E, query_rope, status);
         if (launched != cudaSuccess) {
             return static_cast<int>(launched);
         }

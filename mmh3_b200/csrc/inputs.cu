@@ -22,10 +22,14 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "sm100.cuh"
 
 namespace mmh3 {
 
 namespace {
+
+using sm100::let_next_kernel_begin;
+using sm100::wait_for_kernels_before;
 
 constexpr int BLOCK_ROWS = 64;
 constexpr int THREADS = 256;
@@ -345,7 +349,8 @@ __global__ void __launch_bounds__(THREADS, (NORMALIZE || QUANTIZE) ? 2 : 4)
     __shared__ __align__(16) uint8_t codes[BLOCK_ROWS][CODES_STRIDE];
     __shared__ __align__(16) float maxima[2][WARPS];
     static_assert(WARPS == 8, "the block maximum reads eight warp maxima as two float4");
-    const int block = blockIdx.x;
+    let_next_kernel_begin();
+    const int block = blockIdx.x + wait_for_kernels_before();
     const int blocks = gridDim.x;
     const int first_head = blockIdx.y * p.heads_per_cta;
     const int head_count = min(p.heads_per_cta, p.heads - first_head);
@@ -710,8 +715,9 @@ __global__ void __launch_bounds__(THREADS, (NORMALIZE || QUANTIZE) ? 2 : 4)
 // (crates/mmh3-cuda/kernels/quantized_attention.cu:116-127).
 __global__ void value_scales_kernel(const float *__restrict__ maxima, float *__restrict__ scales,
                                     int blocks) {
+    let_next_kernel_begin();
     float maximum = 0.0f;
-    for (int block = threadIdx.x; block < blocks; block += blockDim.x) {
+    for (int block = threadIdx.x + wait_for_kernels_before(); block < blocks; block += blockDim.x) {
         maximum = fmaxf(maximum, maxima[static_cast<size_t>(blockIdx.x) * blocks + block]);
     }
     __shared__ float partial[32];
@@ -746,8 +752,8 @@ int launch_as(const InputsParams &params, int blocks, size_t shared, cudaStream_
         }
     }
     const int groups = (params.heads + params.heads_per_cta - 1) / params.heads_per_cta;
-    kernel<<<dim3(blocks, groups), THREADS, shared, stream>>>(params);
-    return static_cast<int>(cudaGetLastError());
+    return static_cast<int>(
+        launch_behind(kernel, dim3(blocks, groups), THREADS, shared, stream, params));
 }
 
 template <bool NORMALIZE, bool STATS, bool QUANTIZE>
@@ -936,9 +942,9 @@ int launch_quantize(const void *query, const void *key, const void *value, int t
             return status;
         }
     }
-    value_scales_kernel<<<heads, 256, 0, stream>>>(workspace.value_maxima, workspace.value_scales,
-                                                   blocks);
-    cudaError_t launched = cudaGetLastError();
+    const cudaError_t launched =
+        launch_behind(value_scales_kernel, dim3(heads), 256, 0, stream, workspace.value_maxima,
+                      workspace.value_scales, blocks);
     if (launched != cudaSuccess) {
         return static_cast<int>(launched);
     }

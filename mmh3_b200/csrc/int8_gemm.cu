@@ -157,6 +157,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
     volatile uint32_t *tmem_slot = &tmem_slot_storage;
     const Watchdog watchdog{abort_flag, status};
     auto barrier = [&](int index) { return smem_u32(&barriers[index]); };
+    let_next_kernel_begin();
     const int warp = warp_index();
     const int lane = threadIdx.x % 32;
     const int tiles = walk.tiles();
@@ -183,6 +184,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
     tcgen05_fence_before();
     __syncthreads();
     cluster_sync();
+    wait_for_kernels_before();
     tcgen05_fence_after();
     const uint32_t tmem = *tmem_slot;
 
@@ -583,11 +585,10 @@ int launch_kernel(const GemmMaps &maps, const float *activation_scales, const fl
         return INVALID_VALUE;
     }
     const int blocks = 2 * (tiles < pairs ? static_cast<int>(tiles) : pairs);
-    int8_gemm_kernel<Output, SWIGLU, ADAPTED><<<blocks, THREADS, SMEM_BYTES, stream>>>(
-        maps, activation_scales, weight_scales, bias, output, m, n, k / BLOCK_K, output_stride,
-        walk, maxima, maxima_first_column, ADAPTED ? rank * 2 / BLOCK_K : 0, adapter_scale,
-        status);
-    return static_cast<int>(cudaGetLastError());
+    return static_cast<int>(launch_behind(
+        int8_gemm_kernel<Output, SWIGLU, ADAPTED>, dim3(blocks), THREADS, SMEM_BYTES, stream, maps,
+        activation_scales, weight_scales, bias, output, m, n, k / BLOCK_K, output_stride, walk,
+        maxima, maxima_first_column, ADAPTED ? rank * 2 / BLOCK_K : 0, adapter_scale, status));
 }
 
 __global__ void interleave_rows_kernel(const uint32_t *__restrict__ source,

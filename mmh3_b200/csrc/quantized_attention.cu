@@ -119,9 +119,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     const Watchdog watchdog = {abort_flag, status};
     auto barrier = [&](int index) { return barriers + index * 8; };
 
-    if (*reinterpret_cast<volatile unsigned int *>(status) != 0) {
-        return;
-    }
+    let_next_kernel_begin();
     const int warp = threadIdx.x / 32;
     const int lane = threadIdx.x % 32;
     const int head = blockIdx.y;
@@ -146,10 +144,18 @@ __global__ void __launch_bounds__(THREADS, 1)
     if (warp == MMA_WARP) {
         tmem_alloc(smem_u32(const_cast<uint32_t *>(tmem_slot)), TMEM_COLUMNS);
     }
+    wait_for_kernels_before();
     tcgen05_fence_before();
-    __syncthreads();
+    // Once a wait has run out anywhere, the rest of the grid drains instead of waiting too.
+    const bool stopped = __syncthreads_or(*reinterpret_cast<volatile unsigned int *>(status) != 0);
     tcgen05_fence_after();
     const uint32_t tmem = *tmem_slot;
+    if (stopped) {
+        if (warp == MMA_WARP) {
+            tmem_dealloc(tmem, TMEM_COLUMNS);
+        }
+        return;
+    }
 
     if (warp >= SOFTMAX_WARPS) {
         register_decrease<OTHER_REGISTERS>();
@@ -527,11 +533,11 @@ int launch_quantized_attention(const Mmh3QuantizedWorkspace &workspace, void *ou
                               layout.token_stride[OUTPUT] % 8 == 0 &&
                               layout.head_stride[OUTPUT] % 8 == 0;
     const dim3 grid((tokens + QUERY_TILES * TILE_M - 1) / (QUERY_TILES * TILE_M), heads);
-    quantized_dense_kernel<<<grid, THREADS, SMEM_BYTES, stream>>>(
-        maps, out, tokens, blocks64, workspace.query_scales, workspace.key_scales,
-        workspace.value_scales, layout.token_stride[OUTPUT], layout.head_stride[OUTPUT],
-        vector_stores, scale * LOG2_E, status);
-    return static_cast<int>(cudaGetLastError());
+    return static_cast<int>(launch_behind(
+        quantized_dense_kernel, grid, THREADS, SMEM_BYTES, stream, maps, out, tokens, blocks64,
+        workspace.query_scales, workspace.key_scales, workspace.value_scales,
+        layout.token_stride[OUTPUT], layout.head_stride[OUTPUT], vector_stores, scale * LOG2_E,
+        status));
 }
 
 } // namespace mmh3

@@ -44,6 +44,28 @@ __device__ __forceinline__ bool elect_one() {
 }
 
 // ---------------------------------------------------------------------------------------------
+// Kernels launched with launch_behind (common.cuh): the next kernel of the stream may be set up
+// once every CTA of this one has begun, and waits here for the kernels before it to have finished
+// and their writes to be visible, before it touches global memory. Every thread waits, so no kernel
+// ends before the ones it was launched behind.
+
+__device__ __forceinline__ void let_next_kernel_begin() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// Returns zero, for an address that a read-only load is to take only after the wait: such loads are
+// not held back by the clobber of memory.
+__device__ __forceinline__ int wait_for_kernels_before() {
+    int zero;
+    asm volatile("griddepcontrol.wait;\n"
+                 "mov.u32 %0, 0;"
+                 : "=r"(zero)
+                 :
+                 : "memory");
+    return zero;
+}
+
+// ---------------------------------------------------------------------------------------------
 // mbarrier
 
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
