@@ -21,9 +21,9 @@
 // tensor memory, two of them, which take turns from tile to tile, so that the MMAs of a tile run
 // while the last one is scaled and stored. Warp 0 of each CTA streams its 128 rows of activations
 // and its half of the weights' 256 columns, 128 bytes of K at a time (32 KB, 128-byte swizzle),
-// through a ring of six with TMA; one thread of warp 1 of the first CTA issues tcgen05.mma
+// through a ring of six (five with an adapter) with TMA; one thread of warp 1 of the first CTA issues tcgen05.mma
 // cta_group::2 kind::i8 of 256 x 256 x 32 over both CTAs' shared memory; eight warps of each CTA
-// scale and round its accumulator, turn their rows around in a staging tile of shared memory so
+// (sixteen with an adapter) scale and round its accumulator, turn their rows around in a staging tile of shared memory so
 // that the stores cover whole 128-byte runs, and give the accumulator back as soon as its last
 // columns are in registers.
 //
@@ -52,18 +52,29 @@ constexpr int BLOCK_K = 128;    // bytes of one stage along K: 128 INT8 values, 
 constexpr int ROWS_BYTES = TILE_M * BLOCK_K;
 constexpr int COLUMNS_BYTES = TILE_N / 2 * BLOCK_K; // the half of the tile's columns a CTA loads
 constexpr int STAGE_BYTES = ROWS_BYTES + COLUMNS_BYTES;
-constexpr int STAGES = 6;
 // Where an epilogue warp turns its 32 rows of 64 columns around for the stores.
 constexpr int STAGING_ROW = 128;
 constexpr int STAGING_BYTES = 32 * STAGING_ROW;
-constexpr int EPILOGUE_WARPS = 8;
-constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + EPILOGUE_WARPS * STAGING_BYTES + 1024;
-static_assert(SMEM_BYTES + 256 <= 227 * 1024, "ring, staging and barriers exceed an SM");
+constexpr int MAX_STAGES = 6;
+
+// A tile's epilogue runs under the next tile's MMAs, except with an adapter, which leaves room for
+// one accumulator: there twice the warps, half the columns each, keep the tensor cores waiting for
+// less (4,213 x 28,672 x 5,376 with SwiGLU: 569 us with eight warps, 526 with sixteen at rank 384,
+// 571 and 543 at rank 64). Their staging tiles cost a stage of the ring.
+template <bool ADAPTED> struct Shape {
+    static constexpr int EPILOGUE_WARPS = ADAPTED ? 16 : 8;
+    static constexpr int STAGES = ADAPTED ? 5 : 6;
+    static constexpr int THREADS = (2 + EPILOGUE_WARPS) * 32;
+    static constexpr int WARP_COLUMNS = TILE_N / (EPILOGUE_WARPS / 4);
+    static constexpr int SMEM_BYTES =
+        STAGES * STAGE_BYTES + EPILOGUE_WARPS * STAGING_BYTES + 1024;
+    static_assert(STAGES <= MAX_STAGES, "more stages than barriers");
+    static_assert(SMEM_BYTES + 256 <= 227 * 1024, "ring, staging and barriers exceed an SM");
+};
 
 constexpr int LOAD_WARP = 0;
 constexpr int MMA_WARP = 1;
 constexpr int FIRST_EPILOGUE_WARP = 2;
-constexpr int THREADS = (FIRST_EPILOGUE_WARP + EPILOGUE_WARPS) * 32;
 constexpr int TMEM_COLUMNS = 2 * TILE_N;
 constexpr uint32_t TMEM_ADAPTER = TILE_N; // the adapter's accumulator, beside the INT32 one
 constexpr int CHUNK = 32; // columns of one tcgen05.ld
@@ -72,8 +83,8 @@ constexpr unsigned int STATUS_GEMM = 0x00040000u;
 
 enum Barrier {
     RING_FULL = 0,
-    RING_EMPTY = RING_FULL + STAGES,
-    ACCUMULATOR_FULL = RING_EMPTY + STAGES, // one per accumulator
+    RING_EMPTY = RING_FULL + MAX_STAGES,
+    ACCUMULATOR_FULL = RING_EMPTY + MAX_STAGES, // one per accumulator
     ACCUMULATOR_EMPTY = ACCUMULATOR_FULL + 2,
     BARRIERS = ACCUMULATOR_EMPTY + 2,
 };
@@ -138,7 +149,7 @@ __device__ __forceinline__ uint32_t gated_pair(Output *output, uint32_t gate_wor
 }
 
 template <typename Output, bool SWIGLU, bool ADAPTED>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Shape<ADAPTED>::THREADS, 1)
     int8_gemm_kernel(const __grid_constant__ GemmMaps maps,
                      const float *__restrict__ activation_scales,
                      const float *__restrict__ weight_scales, const float *__restrict__ bias,
@@ -148,6 +159,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
     // Accumulators of 256 columns that take turns from tile to tile: the adapter's sum takes the
     // second one's columns.
     constexpr int ACCUMULATORS = ADAPTED ? 1 : 2;
+    constexpr int STAGES = Shape<ADAPTED>::STAGES;
+    constexpr int EPILOGUE_WARPS = Shape<ADAPTED>::EPILOGUE_WARPS;
+    constexpr int WARP_COLUMNS = Shape<ADAPTED>::WARP_COLUMNS;
     extern __shared__ uint8_t shared_raw[];
     __shared__ __align__(8) uint64_t barriers[BARRIERS];
     __shared__ uint32_t tmem_slot_storage;
@@ -298,7 +312,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
         const int epilogue_warp = warp - FIRST_EPILOGUE_WARP;
         // A warp reads the quarter of the lanes of tensor memory its number selects.
         const int quarter = warp % 4;
-        const int column_half = epilogue_warp / 4;
+        const int column_part = epilogue_warp / 4;
         const uint32_t lane_base = static_cast<uint32_t>(quarter * 32) << 16;
         uint8_t *staging = shared_raw + (base - smem_u32(shared_raw)) + STAGES * STAGE_BYTES +
                            epilogue_warp * STAGING_BYTES;
@@ -309,18 +323,19 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
             int tile_m, tile_n;
             walk.locate(tile, tile_m, tile_n);
             const int first_row = tile_m * PAIR_M + rank * TILE_M + quarter * 32;
-            // The warp's 128 columns lie in one group of 128.
-            const int first_column = tile_n * TILE_N + column_half * (TILE_N / 2);
+            // The warp's columns lie in one group of 128.
+            const int first_column = tile_n * TILE_N + column_part * WARP_COLUMNS;
             const bool inside = first_column < n;
             const bool track =
                 !SWIGLU && maxima != nullptr && inside && first_column >= maxima_first_column;
             // While the MMAs run: this warp's column scales, bias and row scales into L1.
             if (inside) {
-                const int line = lane % 4;
+                constexpr int LINES = WARP_COLUMNS / 32;
+                const int line = lane % LINES;
                 const void *wanted = nullptr;
-                if (lane < 4) {
+                if (lane < LINES) {
                     wanted = weight_scales + first_column + line * 32;
-                } else if (lane < 8 && bias != nullptr) {
+                } else if (lane < 2 * LINES && bias != nullptr) {
                     wanted = bias + first_column + line * 32;
                 } else if (lane == 8 && first_row < m) {
                     wanted = activation_scales + first_row;
@@ -337,7 +352,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
             }
             tcgen05_fence_after();
             auto accumulator = [&](int chunk) {
-                return tmem + lane_base + buffer * TILE_N + column_half * (TILE_N / 2) +
+                return tmem + lane_base + buffer * TILE_N + column_part * WARP_COLUMNS +
                        chunk * CHUNK;
             };
             auto release = [&]() {
@@ -459,11 +474,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
             if constexpr (ADAPTED) {
                 // The product and the adapter's sum of the same 32 columns, side by side.
                 #pragma unroll
-                for (int chunk = 0; chunk < TILE_N / 2 / CHUNK; chunk++) {
+                for (int chunk = 0; chunk < WARP_COLUMNS / CHUNK; chunk++) {
                     tmem_load_32(accumulator(chunk), even);
                     tmem_load_32(accumulator(chunk) + TMEM_ADAPTER, odd);
                     tmem_wait_load();
-                    if (chunk == TILE_N / 2 / CHUNK - 1) {
+                    if (chunk == WARP_COLUMNS / CHUNK - 1) {
                         release();
                     }
                     if (!idle) {
@@ -531,7 +546,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
 // How many pairs of CTAs of `kernel` the device holds at once, asked for once per device.
 struct ResidentPairs {
     std::atomic<int> counts[MAX_DEVICES];
-    template <typename Kernel> int ask(Kernel kernel) {
+    template <typename Kernel> int ask(Kernel kernel, int threads, int shared_bytes) {
         const int device = current_device();
         if (device < 0) {
             return 0;
@@ -546,8 +561,8 @@ struct ResidentPairs {
         cluster.val.clusterDim.z = 1;
         cudaLaunchConfig_t configuration = {};
         configuration.gridDim = dim3(2);
-        configuration.blockDim = dim3(THREADS);
-        configuration.dynamicSmemBytes = SMEM_BYTES;
+        configuration.blockDim = dim3(threads);
+        configuration.dynamicSmemBytes = shared_bytes;
         configuration.attrs = &cluster;
         configuration.numAttrs = 1;
         int pairs = 0;
@@ -564,6 +579,8 @@ int launch_kernel(const GemmMaps &maps, const float *activation_scales, const fl
                   const float *bias, Output *output, int m, int n, int k, int output_stride,
                   int band, unsigned *maxima, int maxima_first_column, int rank,
                   float adapter_scale, cudaStream_t stream) {
+    constexpr int THREADS = Shape<ADAPTED>::THREADS;
+    constexpr int SMEM_BYTES = Shape<ADAPTED>::SMEM_BYTES;
     unsigned int *status = status_pointer();
     static SharedMemoryOptIn shared_memory;
     static ResidentPairs resident;
@@ -572,7 +589,7 @@ int launch_kernel(const GemmMaps &maps, const float *activation_scales, const fl
     if (configured != cudaSuccess) {
         return static_cast<int>(configured);
     }
-    const int pairs = resident.ask(int8_gemm_kernel<Output, SWIGLU, ADAPTED>);
+    const int pairs = resident.ask(int8_gemm_kernel<Output, SWIGLU, ADAPTED>, THREADS, SMEM_BYTES);
     if (status == nullptr || pairs == 0) {
         return static_cast<int>(cudaErrorInvalidDevice);
     }
