@@ -119,11 +119,15 @@ template <bool HALF, int DIM = 128> struct Element {
 
 // The maximum may lag the true row maximum by this much (in log2 units) before O is rescaled.
 constexpr float RESCALE_THRESHOLD = 8.0f;
-// Of every four pairs of probabilities, how many take the polynomial exp2 instead of the MUFU.
-// One in four costs fewer cycles a block (3,466 against 3,543) and more power: over the twenty
-// launches of a benchmark run the GPU sits at its power cap, where none in four runs at 1,627 MHz
-// instead of 1,582 and is the faster by 0.6 % (2 % in the token attention over routes).
-constexpr int POLYNOMIAL_PAIRS_OF_4 = 0;
+// Of every eight pairs of probabilities, how many take the polynomial exp2 instead of the MUFU. With
+// heads of 64 the MMAs are half as long and the exponentials bound a block: eight windows of 1,025
+// tokens with 16 heads take 137.2 us with none, 131.9 with two, 131.3 with three and 142.5 with four
+// (the FMA pipe is then the fuller one); looking for NaNs, which the polynomial has none of, makes
+// 133.5 of three. The error against 64 bits stays at 3.58e-4 (FP16). With
+// heads of 128 two of eight cost fewer cycles a block (3,466 against 3,543) and more power: over
+// the twenty launches of a benchmark run the GPU sits at its power cap, where none runs at 1,627
+// MHz instead of 1,582 and is the faster by 0.6 % (2 % in the token attention over routes).
+template <int DIM> constexpr int POLYNOMIAL_PAIRS_OF_8 = DIM == 64 ? 3 : 0;
 
 struct DenseMaps {
     CUtensorMap query;
@@ -518,13 +522,22 @@ __global__ void __launch_bounds__(THREADS, 1)
                     }
                 }
             }
+            // The polynomial has no NaN to give: where it is used, a score that is one, or plus
+            // infinity, shows in the maximum and goes into the sum by which the row is divided.
+            constexpr bool WATCHED = POLYNOMIAL_PAIRS_OF_8<DIM> > 0;
+            auto larger = [](float first, float second) {
+                return WATCHED ? max_or_nan(first, second) : fmaxf(first, second);
+            };
             float partial[4] = {s[0], s[1], s[2], s[3]};
             #pragma unroll
             for (int index = 4; index < TILE_N; index++) {
-                partial[index % 4] = fmaxf(partial[index % 4], s[index]);
+                partial[index % 4] = larger(partial[index % 4], s[index]);
             }
             const float block_maximum =
-                fmaxf(fmaxf(partial[0], partial[1]), fmaxf(partial[2], partial[3]));
+                larger(larger(partial[0], partial[1]), larger(partial[2], partial[3]));
+            if (WATCHED && !(block_maximum < INFINITY)) {
+                sums[0].x = NAN;
+            }
             if (block == 0) {
                 maximum = block_maximum;
             } else {
@@ -553,7 +566,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                 }
             }
             // p = 2^(s * scale - maximum * scale), two elements at a time, on the MUFU (or a share
-            // of the pairs on the FMA pipe's polynomial, see POLYNOMIAL_PAIRS_OF_4).
+            // of the pairs, spread evenly, on the FMA pipe's polynomial: POLYNOMIAL_PAIRS_OF_8).
             const float offset = maximum * scale_log2;
             const float2 scale2 = make_float2(scale_log2, scale_log2);
             const float2 offset2 = make_float2(-offset, -offset);
@@ -566,7 +579,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                     const float2 x =
                         __ffma2_rn(make_float2(s[index], s[index + 1]), scale2, offset2);
                     float2 probability;
-                    if (pair % 4 < POLYNOMIAL_PAIRS_OF_4) {
+                    if (pair * 3 % 8 < POLYNOMIAL_PAIRS_OF_8<DIM>) {
                         probability = exp2_polynomial(x);
                     } else {
                         probability = make_float2(exp2_approx(x.x), exp2_approx(x.y));

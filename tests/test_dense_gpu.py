@@ -383,6 +383,38 @@ def test_fused_query_rope_against_float64(element_type, head_dim, tokens, pairs)
     assert torch.max(torch.abs(ours.cpu().double() - expected)) <= 2e-2
 
 
+@pytest.mark.parametrize("element_type", [0, 1])
+def test_heads_of_64_whose_exponentials_come_two_ways(element_type):
+    """Three of eight pairs of keys take a polynomial: every key alone in turn holds a row's weight or a
+    NaN, and scores far below the maximum weigh nothing."""
+    tokens, heads, head_dim = 128, 2, 64
+    dtype = torch.float16 if element_type == 1 else torch.bfloat16
+    layout = attention.make_layout((heads * head_dim,) * 4, head_stride=(head_dim,) * 4)
+    q = torch.zeros((tokens, heads, head_dim))
+    k = torch.zeros_like(q)
+    # Row i points at key i: 60 * 8 / 8 above the others, 2^-86 of the weight left to them.
+    for row in range(tokens):
+        q[row, :, row // 2] = 60.0
+        k[row, :, row // 2] = 8.0 if row % 2 else -8.0
+    q[0::2] = -q[0::2]
+    v = torch.randn(q.shape, generator=torch.Generator().manual_seed(1))
+
+    def run(key):
+        output = torch.zeros(q.shape, dtype=dtype, device="cuda")
+        attention.attention(element_type, head_dim, q.to(dtype).cuda(), key.to(dtype).cuda(),
+                            v.to(dtype).cuda(), output, tokens, heads, 1, layout, 0.125)
+        assert attention.take_status() == 0
+        return output.cpu().float()
+
+    # One probability of one, whose value is then the output to the bit.
+    assert torch.equal(run(k), v.to(dtype).float())
+    for column in (0, 1, 6, 7, 12, 13, 127):
+        poisoned = k.clone()
+        poisoned[column, 0, 0] = float("nan")
+        result = run(poisoned)
+        assert torch.isnan(result[:, 0]).all() and torch.isfinite(result[:, 1]).all()
+
+
 def test_unsupported_combinations_report_an_error():
     tokens, heads = 64, 1
     qkv = torch.zeros((tokens, 3, heads, 128), dtype=torch.bfloat16, device="cuda")
