@@ -21,20 +21,20 @@
 // tensor memory, two of them, which take turns from tile to tile, so that the MMAs of a tile run
 // while the last one is scaled and stored. Warp 0 of each CTA streams its 128 rows of activations
 // and its half of the weights' 256 columns, 128 bytes of K at a time (32 KB, 128-byte swizzle),
-// through a ring of six (five with an adapter) with TMA; one thread of warp 1 of the first CTA issues tcgen05.mma
-// cta_group::2 kind::i8 of 256 x 256 x 32 over both CTAs' shared memory; eight warps of each CTA
-// (sixteen with an adapter) scale and round its accumulator, turn their rows around in a staging tile of shared memory so
-// that the stores cover whole 128-byte runs, and give the accumulator back as soon as its last
-// columns are in registers.
+// through a ring of six (five with an adapter) with TMA; one thread of warp 1 of the first CTA
+// issues tcgen05.mma cta_group::2 kind::i8 of 256 x 256 x 32 over both CTAs' shared memory; eight
+// warps of each CTA (sixteen with an adapter) scale and round its accumulator, turn their rows around
+// in a staging tile of shared memory so that the stores cover whole 128-byte runs, and give the
+// accumulator back as soon as its last columns are in registers. Few tiles go to single CTAs of 128
+// rows instead: launch_kernel says when.
 //
 // What bounds it is the MMAs and, in a long run, the power they draw. The pair is what hides the
 // epilogue: an SM takes 32 KB per 512 cycles of MMA from L2, 64 bytes a cycle, about what it can
-// get; one CTA alone with 128 x 256 tiles and two accumulators would need 96, and with tiles of 256
-// x 256 (64 bytes a cycle, no second accumulator) the tensor cores waited for an epilogue of about
-// 12,000 cycles in every 46,000. Against that kernel, whole calls: a SwiGLU layer of 4,213 x 28,672
-// x 5,376 with an adapter of rank 384 went from 710 us to 672 (an adapter leaves no room for the
-// second accumulator, but its 128-row tiles took the 96 bytes a cycle), a DiT attention layer of
-// 16,896 tokens, whose qkv projection is a fifth of it, from 7.70 ms to 7.52.
+// get; one CTA alone with 128 x 256 tiles and two accumulators needs 96, and with tiles of 256 x 256
+// (64 bytes a cycle, no second accumulator) the tensor cores waited for an epilogue of about
+// 12,000 cycles in every 46,000. Against that kernel: 66,048 x 12,288 x 4,096 went from 2.30 ms to
+// 2.03, 4,213 x 28,672 x 5,376 with SwiGLU from 558 us to 515, and with an adapter of rank 384 (no
+// room for the second accumulator, but its 128-row tiles took the 96 bytes a cycle) from 636 us to 570.
 #include "common.cuh"
 #include "sm100.cuh"
 
@@ -45,13 +45,10 @@ namespace {
 
 using namespace sm100;
 
-constexpr int TILE_M = 128;     // rows of a tile in one CTA of the pair
-constexpr int PAIR_M = 2 * TILE_M;
+constexpr int TILE_M = 128;     // rows of a tile in one CTA
 constexpr int TILE_N = 256;
 constexpr int BLOCK_K = 128;    // bytes of one stage along K: 128 INT8 values, 64 BF16 ranks
 constexpr int ROWS_BYTES = TILE_M * BLOCK_K;
-constexpr int COLUMNS_BYTES = TILE_N / 2 * BLOCK_K; // the half of the tile's columns a CTA loads
-constexpr int STAGE_BYTES = ROWS_BYTES + COLUMNS_BYTES;
 // Where an epilogue warp turns its 32 rows of 64 columns around for the stores.
 constexpr int STAGING_ROW = 128;
 constexpr int STAGING_BYTES = 32 * STAGING_ROW;
@@ -61,13 +58,21 @@ constexpr int MAX_STAGES = 6;
 // one accumulator: there twice the warps, half the columns each, keep the tensor cores waiting for
 // less (4,213 x 28,672 x 5,376 with SwiGLU: 569 us with eight warps, 526 with sixteen at rank 384,
 // 571 and 543 at rank 64). Their staging tiles cost a stage of the ring.
-template <bool ADAPTED> struct Shape {
-    static constexpr int EPILOGUE_WARPS = ADAPTED ? 16 : 8;
-    static constexpr int STAGES = ADAPTED ? 5 : 6;
+template <bool ADAPTED, bool PAIR> struct Shape {
+    static constexpr int CTAS = PAIR ? 2 : 1; // that share a tile
+    static constexpr int TILE_ROWS = CTAS * TILE_M;
+    static constexpr int LOADED_COLUMNS = TILE_N / CTAS; // a CTA's share of the tile's columns
+    static constexpr int STAGE_BYTES = ROWS_BYTES + LOADED_COLUMNS * BLOCK_K;
+    static constexpr int EPILOGUE_WARPS = ADAPTED && PAIR ? 16 : 8;
+    static constexpr int STAGES = PAIR ? (ADAPTED ? 5 : 6) : 4;
     static constexpr int THREADS = (2 + EPILOGUE_WARPS) * 32;
     static constexpr int WARP_COLUMNS = TILE_N / (EPILOGUE_WARPS / 4);
     static constexpr int SMEM_BYTES =
         STAGES * STAGE_BYTES + EPILOGUE_WARPS * STAGING_BYTES + 1024;
+    static constexpr uint32_t PRODUCT_MMA =
+        instruction_descriptor(ACCUMULATE_S32, FORMAT_S8, FORMAT_S8, 0, 0, TILE_ROWS, TILE_N);
+    static constexpr uint32_t ADAPTER_MMA =
+        instruction_descriptor(ACCUMULATE_F32, FORMAT_BF16, FORMAT_BF16, 0, 0, TILE_ROWS, TILE_N);
     static_assert(STAGES <= MAX_STAGES, "more stages than barriers");
     static_assert(SMEM_BYTES + 256 <= 227 * 1024, "ring, staging and barriers exceed an SM");
 };
@@ -88,12 +93,6 @@ enum Barrier {
     ACCUMULATOR_EMPTY = ACCUMULATOR_FULL + 2,
     BARRIERS = ACCUMULATOR_EMPTY + 2,
 };
-
-constexpr uint32_t PRODUCT_MMA =
-    instruction_descriptor(ACCUMULATE_S32, FORMAT_S8, FORMAT_S8, 0, 0, PAIR_M, TILE_N);
-
-constexpr uint32_t ADAPTER_MMA =
-    instruction_descriptor(ACCUMULATE_F32, FORMAT_BF16, FORMAT_BF16, 0, 0, PAIR_M, TILE_N);
 
 struct GemmMaps {
     CUtensorMap activations;  // [m, k] INT8
@@ -148,8 +147,9 @@ __device__ __forceinline__ uint32_t gated_pair(Output *output, uint32_t gate_wor
                                     gate.y / (1.0f + __expf(-gate.y)) * up.y));
 }
 
-template <typename Output, bool SWIGLU, bool ADAPTED>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Shape<ADAPTED>::THREADS, 1)
+template <typename Output, bool SWIGLU, bool ADAPTED, bool PAIR>
+__global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1)
+    __launch_bounds__(Shape<ADAPTED, PAIR>::THREADS, 1)
     int8_gemm_kernel(const __grid_constant__ GemmMaps maps,
                      const float *__restrict__ activation_scales,
                      const float *__restrict__ weight_scales, const float *__restrict__ bias,
@@ -159,9 +159,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Shape<ADAPTED>::THRE
     // Accumulators of 256 columns that take turns from tile to tile: the adapter's sum takes the
     // second one's columns.
     constexpr int ACCUMULATORS = ADAPTED ? 1 : 2;
-    constexpr int STAGES = Shape<ADAPTED>::STAGES;
-    constexpr int EPILOGUE_WARPS = Shape<ADAPTED>::EPILOGUE_WARPS;
-    constexpr int WARP_COLUMNS = Shape<ADAPTED>::WARP_COLUMNS;
+    using S = Shape<ADAPTED, PAIR>;
+    constexpr int CTAS = S::CTAS;
+    constexpr int STAGES = S::STAGES;
+    constexpr int STAGE_BYTES = S::STAGE_BYTES;
+    constexpr int EPILOGUE_WARPS = S::EPILOGUE_WARPS;
+    constexpr int WARP_COLUMNS = S::WARP_COLUMNS;
     extern __shared__ uint8_t shared_raw[];
     __shared__ __align__(8) uint64_t barriers[BARRIERS];
     __shared__ uint32_t tmem_slot_storage;
@@ -175,9 +178,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Shape<ADAPTED>::THRE
     const int warp = warp_index();
     const int lane = threadIdx.x % 32;
     const int tiles = walk.tiles();
-    const int rank = static_cast<int>(cluster_rank()); // the CTA of the pair; the first issues the MMAs
-    const int first_tile = blockIdx.x / 2;
-    const int tile_step = gridDim.x / 2;
+    // The CTA of the pair; the first issues the MMAs.
+    const int rank = PAIR ? static_cast<int>(cluster_rank()) : 0;
+    const int first_tile = blockIdx.x / CTAS;
+    const int tile_step = gridDim.x / CTAS;
+    auto commit = [&](int index) {
+        if constexpr (PAIR) {
+            tcgen05_commit_pair(barrier(index));
+        } else {
+            tcgen05_commit(barrier(index));
+        }
+    };
 
     if (threadIdx.x == 0) {
         for (int stage = 0; stage < STAGES; stage++) {
@@ -186,18 +197,24 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Shape<ADAPTED>::THRE
         }
         for (int buffer = 0; buffer < ACCUMULATORS; buffer++) {
             mbar_init(barrier(ACCUMULATOR_FULL + buffer), 1);
-            mbar_init(barrier(ACCUMULATOR_EMPTY + buffer), 2 * EPILOGUE_WARPS);
+            mbar_init(barrier(ACCUMULATOR_EMPTY + buffer), CTAS * EPILOGUE_WARPS);
         }
         *abort_flag = 0;
         fence_barrier_init();
         fence_proxy_async();
     }
     if (warp == MMA_WARP) {
-        tmem_alloc_pair(smem_u32(const_cast<uint32_t *>(tmem_slot)), TMEM_COLUMNS);
+        if constexpr (PAIR) {
+            tmem_alloc_pair(smem_u32(const_cast<uint32_t *>(tmem_slot)), TMEM_COLUMNS);
+        } else {
+            tmem_alloc(smem_u32(const_cast<uint32_t *>(tmem_slot)), TMEM_COLUMNS);
+        }
     }
     tcgen05_fence_before();
     __syncthreads();
-    cluster_sync();
+    if constexpr (PAIR) {
+        cluster_sync();
+    }
     wait_for_kernels_before();
     tcgen05_fence_after();
     const uint32_t tmem = *tmem_slot;
@@ -215,8 +232,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Shape<ADAPTED>::THRE
             for (int tile = first_tile; alive && tile < tiles; tile += tile_step) {
                 int tile_m, tile_n;
                 walk.locate(tile, tile_m, tile_n);
-                const int row = tile_m * PAIR_M + rank * TILE_M;
-                const int column = tile_n * TILE_N + rank * (TILE_N / 2);
+                const int row = tile_m * S::TILE_ROWS + rank * TILE_M;
+                const int column = tile_n * TILE_N + rank * S::LOADED_COLUMNS;
                 // The K blocks of the INT8 operands, then the adapter's blocks of 64 ranks: the
                 // same 128-byte rows in the same places. The bytes of both CTAs are counted by the
                 // first one's barrier, which expects them all.
@@ -229,24 +246,28 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Shape<ADAPTED>::THRE
                         break;
                     }
                     const uint32_t destination = base + stage * STAGE_BYTES;
-                    const uint32_t full = cluster_address(barrier(RING_FULL + stage), 0);
                     const bool adapter = block >= k_blocks;
                     // Coordinates are in elements: bytes for INT8, BF16 values for the adapter.
                     const int along = adapter ? (block - k_blocks) * (BLOCK_K / 2) : block * BLOCK_K;
+                    const CUtensorMap *rows_map = adapter ? &maps.adapter_down : &maps.activations;
+                    const CUtensorMap *columns_map = adapter ? &maps.adapter_up : &maps.weights;
                     if (rank == 0) {
-                        mbar_expect_tx(barrier(RING_FULL + stage), 2 * STAGE_BYTES);
+                        mbar_expect_tx(barrier(RING_FULL + stage), CTAS * STAGE_BYTES);
                     }
-                    tma_load_2d_pair(destination,
-                                     adapter ? &maps.adapter_down : &maps.activations, full, along,
-                                     row);
-                    tma_load_2d_pair(destination + ROWS_BYTES,
-                                     adapter ? &maps.adapter_up : &maps.weights, full, along,
-                                     column);
+                    if constexpr (PAIR) {
+                        const uint32_t full = cluster_address(barrier(RING_FULL + stage), 0);
+                        tma_load_2d_pair(destination, rows_map, full, along, row);
+                        tma_load_2d_pair(destination + ROWS_BYTES, columns_map, full, along, column);
+                    } else {
+                        const uint32_t full = barrier(RING_FULL + stage);
+                        tma_load_2d(destination, rows_map, full, along, row);
+                        tma_load_2d(destination + ROWS_BYTES, columns_map, full, along, column);
+                    }
                 }
             }
-            // The commits of the last uses arrive here from the first CTA: they do before this CTA
-            // may leave.
-            for (int last = item - 1; alive && last >= 0 && last >= item - STAGES; last--) {
+            // The commits of the last uses arrive here from the pair's first CTA: they do before this
+            // CTA may leave.
+            for (int last = item - 1; PAIR && alive && last >= 0 && last >= item - STAGES; last--) {
                 alive = mbar_wait(barrier(RING_EMPTY + last % STAGES), last / STAGES & 1, watchdog,
                                   STATUS_GEMM | 5);
             }
@@ -261,9 +282,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Shape<ADAPTED>::THRE
                 const uint64_t columns = smem_descriptor(stage_base + ROWS_BYTES, 16, 1024);
                 #pragma unroll
                 for (int step = 0; step < BLOCK_K / 32; step++) {
-                    mma_i8_pair_ss(accumulator, advance_descriptor(rows, step * 32),
-                                   advance_descriptor(columns, step * 32), PRODUCT_MMA,
-                                   !first || step > 0);
+                    const uint64_t a = advance_descriptor(rows, step * 32);
+                    const uint64_t b = advance_descriptor(columns, step * 32);
+                    if constexpr (PAIR) {
+                        mma_i8_pair_ss(accumulator, a, b, S::PRODUCT_MMA, !first || step > 0);
+                    } else {
+                        mma_i8_ss(accumulator, a, b, S::PRODUCT_MMA, !first || step > 0);
+                    }
                 }
             };
             auto adapt = [&](int stage, bool first) {
@@ -272,9 +297,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Shape<ADAPTED>::THRE
                 const uint64_t columns = smem_descriptor(stage_base + ROWS_BYTES, 16, 1024);
                 #pragma unroll
                 for (int step = 0; step < BLOCK_K / 32; step++) {
-                    mma_f16_pair_ss(tmem + TMEM_ADAPTER, advance_descriptor(rows, step * 32),
-                                    advance_descriptor(columns, step * 32), ADAPTER_MMA,
-                                    !first || step > 0);
+                    const uint64_t a = advance_descriptor(rows, step * 32);
+                    const uint64_t b = advance_descriptor(columns, step * 32);
+                    if constexpr (PAIR) {
+                        mma_f16_pair_ss(tmem + TMEM_ADAPTER, a, b, S::ADAPTER_MMA,
+                                        !first || step > 0);
+                    } else {
+                        mma_f16_ss(tmem + TMEM_ADAPTER, a, b, S::ADAPTER_MMA, !first || step > 0);
+                    }
                 }
             };
             int item = 0;
@@ -301,10 +331,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Shape<ADAPTED>::THRE
                     } else {
                         multiply(tmem + buffer * TILE_N, stage, block == 0);
                     }
-                    tcgen05_commit_pair(barrier(RING_EMPTY + stage));
+                    commit(RING_EMPTY + stage);
                 }
                 if (alive) {
-                    tcgen05_commit_pair(barrier(ACCUMULATOR_FULL + buffer));
+                    commit(ACCUMULATOR_FULL + buffer);
                 }
             }
         }
@@ -322,7 +352,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Shape<ADAPTED>::THRE
             const int buffer = round % ACCUMULATORS;
             int tile_m, tile_n;
             walk.locate(tile, tile_m, tile_n);
-            const int first_row = tile_m * PAIR_M + rank * TILE_M + quarter * 32;
+            const int first_row = tile_m * S::TILE_ROWS + rank * TILE_M + quarter * 32;
             // The warp's columns lie in one group of 128.
             const int first_column = tile_n * TILE_N + column_part * WARP_COLUMNS;
             const bool inside = first_column < n;
@@ -359,7 +389,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Shape<ADAPTED>::THRE
                 tcgen05_fence_before();
                 __syncwarp();
                 if (lane == 0) {
-                    mbar_arrive_cluster(cluster_address(barrier(ACCUMULATOR_EMPTY + buffer), 0));
+                    if constexpr (PAIR) {
+                        mbar_arrive_cluster(
+                            cluster_address(barrier(ACCUMULATOR_EMPTY + buffer), 0));
+                    } else {
+                        mbar_arrive(barrier(ACCUMULATOR_EMPTY + buffer));
+                    }
                 }
             };
             // Two buffers take turns: the load of the next 32 columns is in flight while these
@@ -535,11 +570,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Shape<ADAPTED>::THRE
         }
     }
     __syncwarp();
-    // Neither CTA leaves while the other may still reach into it.
-    cluster_sync();
+    if constexpr (PAIR) {
+        // Neither CTA leaves while the other may still reach into it.
+        cluster_sync();
+    }
     if (warp == MMA_WARP) {
         tcgen05_fence_after();
-        tmem_dealloc_pair(tmem, TMEM_COLUMNS);
+        if constexpr (PAIR) {
+            tmem_dealloc_pair(tmem, TMEM_COLUMNS);
+        } else {
+            tmem_dealloc(tmem, TMEM_COLUMNS);
+        }
     }
 }
 
@@ -574,38 +615,117 @@ struct ResidentPairs {
     }
 };
 
-template <typename Output, bool SWIGLU, bool ADAPTED>
-int launch_kernel(const GemmMaps &maps, const float *activation_scales, const float *weight_scales,
-                  const float *bias, Output *output, int m, int n, int k, int output_stride,
-                  int band, unsigned *maxima, int maxima_first_column, int rank,
-                  float adapter_scale, cudaStream_t stream) {
-    constexpr int THREADS = Shape<ADAPTED>::THREADS;
-    constexpr int SMEM_BYTES = Shape<ADAPTED>::SMEM_BYTES;
-    unsigned int *status = status_pointer();
-    static SharedMemoryOptIn shared_memory;
+// The pairs of CTAs that take turns at the tiles of 256 rows, or 0 if the device cannot say.
+template <typename Output, bool SWIGLU, bool ADAPTED> int resident_pairs() {
+    using S = Shape<ADAPTED, true>;
     static ResidentPairs resident;
-    const cudaError_t configured =
-        shared_memory.ensure(int8_gemm_kernel<Output, SWIGLU, ADAPTED>, SMEM_BYTES);
+    static SharedMemoryOptIn shared_memory;
+    const auto kernel = int8_gemm_kernel<Output, SWIGLU, ADAPTED, true>;
+    if (shared_memory.ensure(kernel, S::SMEM_BYTES) != cudaSuccess) {
+        return 0;
+    }
+    return resident.ask(kernel, S::THREADS, S::SMEM_BYTES);
+}
+
+struct GemmTask {
+    const int8_t *activations;
+    const int8_t *weights;
+    const float *activation_scales;
+    const float *weight_scales;
+    const float *bias;
+    void *output;
+    int m, n, k, output_stride, band;
+    const void *adapter_down;
+    const void *adapter_up;
+    int rank, adapter_down_stride;
+    float adapter_scale;
+    unsigned *maxima;
+    int maxima_first_column;
+};
+
+template <typename Output, bool SWIGLU, bool ADAPTED, bool PAIR>
+int launch_tiles(const GemmTask &task, int in_flight, cudaStream_t stream) {
+    using S = Shape<ADAPTED, PAIR>;
+    unsigned int *status = status_pointer();
+    if (status == nullptr || in_flight == 0) {
+        return static_cast<int>(cudaErrorInvalidDevice);
+    }
+    const auto kernel = int8_gemm_kernel<Output, SWIGLU, ADAPTED, PAIR>;
+    static SharedMemoryOptIn shared_memory;
+    const cudaError_t configured = shared_memory.ensure(kernel, S::SMEM_BYTES);
     if (configured != cudaSuccess) {
         return static_cast<int>(configured);
     }
-    const int pairs = resident.ask(int8_gemm_kernel<Output, SWIGLU, ADAPTED>, THREADS, SMEM_BYTES);
-    if (status == nullptr || pairs == 0) {
-        return static_cast<int>(cudaErrorInvalidDevice);
+    GemmMaps maps;
+    const uint64_t m = static_cast<uint64_t>(task.m), n = static_cast<uint64_t>(task.n);
+    const uint64_t k = static_cast<uint64_t>(task.k), rank = static_cast<uint64_t>(task.rank);
+    const uint64_t row_dimensions[2] = {k, m};
+    const uint64_t column_dimensions[2] = {k, n};
+    const uint64_t strides[1] = {k};
+    const uint32_t row_box[2] = {BLOCK_K, TILE_M};
+    const uint32_t column_box[2] = {BLOCK_K, S::LOADED_COLUMNS};
+    if (!encode_tensor_map(&maps.activations, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, task.activations,
+                           row_dimensions, strides, row_box) ||
+        !encode_tensor_map(&maps.weights, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, task.weights,
+                           column_dimensions, strides, column_box)) {
+        return INVALID_VALUE;
+    }
+    maps.adapter_down = maps.activations;
+    maps.adapter_up = maps.weights;
+    if constexpr (ADAPTED) {
+        const uint64_t down_dimensions[2] = {rank, m};
+        const uint64_t up_dimensions[2] = {rank, n};
+        const uint64_t down_strides[1] = {static_cast<uint64_t>(task.adapter_down_stride) * 2};
+        const uint64_t up_strides[1] = {rank * 2};
+        const uint32_t down_box[2] = {BLOCK_K / 2, TILE_M};
+        const uint32_t up_box[2] = {BLOCK_K / 2, S::LOADED_COLUMNS};
+        if (!encode_tensor_map(&maps.adapter_down, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2,
+                               task.adapter_down, down_dimensions, down_strides, down_box) ||
+            !encode_tensor_map(&maps.adapter_up, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2,
+                               task.adapter_up, up_dimensions, up_strides, up_box)) {
+            return INVALID_VALUE;
+        }
     }
     TileWalk walk;
-    walk.tiles_m = (m + PAIR_M - 1) / PAIR_M;
-    walk.tiles_n = (n + TILE_N - 1) / TILE_N;
-    walk.band = band;
+    walk.tiles_m = (task.m + S::TILE_ROWS - 1) / S::TILE_ROWS;
+    walk.tiles_n = (task.n + TILE_N - 1) / TILE_N;
+    walk.band = task.band;
     const int64_t tiles = static_cast<int64_t>(walk.tiles_m) * walk.tiles_n;
     if (tiles > INT32_MAX) {
         return INVALID_VALUE;
     }
-    const int blocks = 2 * (tiles < pairs ? static_cast<int>(tiles) : pairs);
+    const int blocks = S::CTAS * (tiles < in_flight ? static_cast<int>(tiles) : in_flight);
     return static_cast<int>(launch_behind(
-        int8_gemm_kernel<Output, SWIGLU, ADAPTED>, dim3(blocks), THREADS, SMEM_BYTES, stream, maps,
-        activation_scales, weight_scales, bias, output, m, n, k / BLOCK_K, output_stride, walk,
-        maxima, maxima_first_column, ADAPTED ? rank * 2 / BLOCK_K : 0, adapter_scale, status));
+        kernel, dim3(blocks), S::THREADS, S::SMEM_BYTES, stream, maps, task.activation_scales,
+        task.weight_scales, task.bias, static_cast<Output *>(task.output), task.m, task.n,
+        task.k / BLOCK_K, task.output_stride, walk, task.maxima, task.maxima_first_column,
+        ADAPTED ? task.rank * 2 / BLOCK_K : 0, task.adapter_scale, status));
+}
+
+// Tiles of 256 rows on pairs of CTAs, or of 128 on single ones where those need few enough rounds of
+// the device. A round is the same MMAs either way, but a single CTA takes 96 bytes a cycle from L2
+// instead of 64 (and with an adapter keeps eight epilogue warps): where both need the same number of
+// rounds pairs are the faster by up to a fifth, and at four rounds to five they are level. Pairs
+// and singles, m x n x k: 800 x 5,376 x 7,168 with an adapter (2 rounds and 1) 43.3 and 27.0 us, 300
+// x 12,288 x 4,096 (2 and 1) 26.2 and 17.6, 600 x 28,672 x 5,376 (5 and 4) 86.2 and 85.8, with an
+// adapter 105.4 and 108.6, 2,000 x 12,288 x 4,096 (6 and 6) 70.8 and 82.8, 1,300 x 21,504 x 7,168 with
+// an adapter (7 and 7) 158.5 and 187.2.
+template <typename Output, bool SWIGLU, bool ADAPTED>
+int launch_kernel(const GemmTask &task, cudaStream_t stream) {
+    const int processors = multiprocessor_count();
+    const int pairs = resident_pairs<Output, SWIGLU, ADAPTED>();
+    if (processors == 0 || pairs == 0) {
+        return static_cast<int>(cudaErrorInvalidDevice);
+    }
+    const int64_t columns = (static_cast<int64_t>(task.n) + TILE_N - 1) / TILE_N;
+    auto rounds = [&](int rows, int in_flight) {
+        return ((task.m + static_cast<int64_t>(rows) - 1) / rows * columns + in_flight - 1) / in_flight;
+    };
+    const int64_t of_pairs = rounds(2 * TILE_M, pairs), of_singles = rounds(TILE_M, processors);
+    if (of_singles * 5 < of_pairs * 4) {
+        return launch_tiles<Output, SWIGLU, ADAPTED, false>(task, processors, stream);
+    }
+    return launch_tiles<Output, SWIGLU, ADAPTED, true>(task, pairs, stream);
 }
 
 __global__ void interleave_rows_kernel(const uint32_t *__restrict__ source,
@@ -658,39 +778,11 @@ int launch_int8_gemm(int config, int group_m, const int8_t *activations, const i
         reinterpret_cast<uintptr_t>(bias) % 8 != 0) {
         return INVALID_VALUE;
     }
-    GemmMaps maps;
-    const uint64_t row_dimensions[2] = {static_cast<uint64_t>(k), static_cast<uint64_t>(m)};
-    const uint64_t column_dimensions[2] = {static_cast<uint64_t>(k), static_cast<uint64_t>(n)};
-    const uint64_t strides[1] = {static_cast<uint64_t>(k)};
-    const uint32_t row_box[2] = {BLOCK_K, TILE_M};
-    const uint32_t column_box[2] = {BLOCK_K, TILE_N / 2};
-    if (!encode_tensor_map(&maps.activations, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, activations,
-                           row_dimensions, strides, row_box) ||
-        !encode_tensor_map(&maps.weights, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, weights,
-                           column_dimensions, strides, column_box)) {
-        return INVALID_VALUE;
-    }
-    maps.adapter_down = maps.activations;
-    maps.adapter_up = maps.weights;
-    if (adapted) {
-        const uint64_t down_dimensions[2] = {static_cast<uint64_t>(rank), static_cast<uint64_t>(m)};
-        const uint64_t up_dimensions[2] = {static_cast<uint64_t>(rank), static_cast<uint64_t>(n)};
-        const uint64_t down_strides[1] = {static_cast<uint64_t>(adapter_down_stride) * 2};
-        const uint64_t up_strides[1] = {static_cast<uint64_t>(rank) * 2};
-        const uint32_t down_box[2] = {BLOCK_K / 2, TILE_M};
-        const uint32_t up_box[2] = {BLOCK_K / 2, TILE_N / 2};
-        if (!encode_tensor_map(&maps.adapter_down, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2,
-                               adapter_down, down_dimensions, down_strides, down_box) ||
-            !encode_tensor_map(&maps.adapter_up, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, adapter_up,
-                               up_dimensions, up_strides, up_box)) {
-            return INVALID_VALUE;
-        }
-    }
-    const int band = config >= 0 ? group_m : 8;
-#define MMH3_GEMM(OUTPUT, SWIGLU, ADAPTED)                                                         \
-    launch_kernel<OUTPUT, SWIGLU, ADAPTED>(                                                        \
-        maps, activation_scales, weight_scales, bias, static_cast<OUTPUT *>(output), m, n, k,      \
-        output_stride, band, column_maxima, maxima_first_column, rank, adapter_scale, stream)
+    const GemmTask task = {activations, weights, activation_scales, weight_scales, bias, output,
+                           m, n, k, output_stride, config >= 0 ? group_m : 8, adapter_down,
+                           adapter_up, rank, adapter_down_stride, adapter_scale, column_maxima,
+                           maxima_first_column};
+#define MMH3_GEMM(OUTPUT, SWIGLU, ADAPTED) launch_kernel<OUTPUT, SWIGLU, ADAPTED>(task, stream)
 #define MMH3_GEMM_OUTPUT(OUTPUT)                                                                   \
     (swiglu ? (adapted ? MMH3_GEMM(OUTPUT, true, true) : MMH3_GEMM(OUTPUT, true, false))           \
             : (adapted ? MMH3_GEMM(OUTPUT, false, true) : MMH3_GEMM(OUTPUT, false, false)))

@@ -113,12 +113,13 @@ def test_matches_the_definition_oracle_and_reference(oracle, reference_kernels, 
     (1, 128, 128),       # one row, a tile of 128 columns, one stage
     (128, 256, 768),     # the second CTA of a pair without rows; as many stages as the ring has
     (129, 384, 896),     # one row for it; one stage more
-    (520, 13184, 128),   # more tiles than pairs of CTAs: an accumulator's second and third tile
-    (513, 13312, 1024),
-    (2305, 7936, 256),
+    # More tiles than pairs of CTAs, an accumulator's second and third tile, on pairs ...
+    (700, 13184, 128), (641, 13312, 1024), (2305, 7936, 256),
+    # ... and on single CTAs, which take fewer rounds of these
+    (300, 12288, 640), (520, 13184, 128), (513, 13312, 1024),
 ])
-def test_tiles_of_cta_pairs(oracle, m, n, k):
-    """Two CTAs share a tile of 256 rows and take turns with two accumulators."""
+def test_tiles_of_pairs_and_of_single_ctas(oracle, m, n, k):
+    """Two CTAs share a tile of 256 rows, or one takes 128, with two accumulators in turn."""
     case = gemm_cases.operands(m, n, k, m + k)
     bits, maxima = run(case, m, n, k, first_column=0)
     expected, expected_maxima = oracle_lib.int8_gemm(oracle, *case, maxima_first_column=0)
@@ -127,9 +128,10 @@ def test_tiles_of_cta_pairs(oracle, m, n, k):
 
 
 @pytest.mark.parametrize("m,n,k,rank", [
-    (1, 128, 128, 64), (129, 384, 640, 128), (513, 13312, 256, 64), (300, 28672, 384, 384),
+    (1, 128, 128, 64), (129, 384, 640, 128), (700, 13312, 256, 64), (512, 28672, 384, 384),
+    (513, 13312, 256, 64), (300, 28672, 384, 384),  # on single CTAs
 ])
-def test_tiles_of_cta_pairs_with_an_adapter(m, n, k, rank):
+def test_tiles_of_pairs_and_of_single_ctas_with_an_adapter(m, n, k, rank):
     # The bounds of test_adds_a_low_rank_adapter.
     case = gemm_cases.operands(m, n, k, m + k)
     down, up = gemm_cases.adapter_operands(m, n, rank, rank, 7)
