@@ -752,7 +752,7 @@ int launch_int8_gemm(int config, int group_m, const int8_t *activations, const i
                      int maxima_first_column, cudaStream_t stream) {
     // crates/mmh3-cuda/kernels/int8_gemm.cu:640-645, 700-712, 720-722: config 0 needs N in
     // multiples of 128 and config 1 of 256; a negative config is the tiling chosen for the shape.
-    // Here every config runs the one tiling, whose results do not depend on it.
+    // Here every config runs the tiling that the sizes choose, whose results do not depend on it.
     // int8_gemm.cu:622-624
     const bool adapted = adapter_down != nullptr && adapter_up != nullptr && adapter_scale != 0.0f;
     if (config > 1 || (config >= 0 && group_m <= 0) || m <= 0 || n <= 0 || k <= 0 ||
