@@ -160,6 +160,39 @@ __device__ __forceinline__ uint64_t value_operand(uint32_t tile) {
 }
 __host__ __device__ constexpr uint32_t value_step(int step) { return step * 16 * 128; }
 
+// The sine (x) and cosine (y) of an angle of at most ANGLE_LIMIT without a branch, so that a thread's
+// several are under way together: Cody and Waite's reduction by n quarter turns, pi/2 in three
+// floats, each step one FMA; polynomials fitted over [-pi/4, pi/4] for the smallest relative error
+// (3.9e-9 and 1.2e-10); the quadrant by n's low bits. At most 1.55 units in the last place off over
+// 20 million angles up to the limit; sincosf is allowed two.
+constexpr float ANGLE_LIMIT = 48000.0f;
+__device__ __forceinline__ float2 sine_and_cosine(float angle) {
+    const float n = rintf(angle * 0.636619772f);
+    float r = fmaf(n, -1.5707963705062866f, angle);
+    r = fmaf(n, 4.371138828673793e-08f, r);
+    r = fmaf(n, 1.7151245100058819e-15f, r);
+    const float z = r * r;
+    float sine = fmaf(z, -0.0001951398007804528f, 0.008332150988280773f);
+    sine = fmaf(z, sine, -0.16666653752326965f);
+    sine = fmaf(r * z, sine, r);
+    float cosine = fmaf(z, 2.4431667043245398e-05f, -0.0013887303648516536f);
+    cosine = fmaf(z, cosine, 0.04166664555668831f);
+    cosine = fmaf(z, cosine, -0.5f);
+    cosine = fmaf(z, cosine, 1.0f);
+    const uint32_t quarter = static_cast<uint32_t>(static_cast<int>(n));
+    const float2 turned = quarter & 1u ? make_float2(cosine, sine) : make_float2(sine, cosine);
+    return make_float2(
+        __uint_as_float(__float_as_uint(turned.x) ^ (quarter << 30 & 0x80000000u)),
+        __uint_as_float(__float_as_uint(turned.y) ^ ((quarter + 1u) << 30 & 0x80000000u)));
+}
+
+// The same of any angle, NaN and infinities among them.
+__device__ __noinline__ float2 sine_and_cosine_of_any(float angle) {
+    float2 result;
+    sincosf(angle, &result.x, &result.y);
+    return result;
+}
+
 template <bool HALF, bool CAUSAL, int DIM, bool ROPE>
 __global__ void __launch_bounds__(THREADS, 1)
     dense_bf16_kernel(const __grid_constant__ DenseMaps maps, uint16_t *__restrict__ output,
@@ -382,75 +415,114 @@ __global__ void __launch_bounds__(THREADS, 1)
             // a warp to a row. A lane takes both dimensions of its pairs, so that nothing crosses
             // lanes but the sum of squares and a pair's sine and cosine are computed once, and then
             // its share of the dimensions behind the pairs. A row alone is a chain of loads,
-            // shuffles and sincosf, so a warp has ROWS_AT_ONCE of them under way: eight windows of
-            // 1,025 tokens with 16 heads of 64 and 32 pairs took 180 us with a row at a time and
-            // every sine and cosine computed twice, and take 138.
-            alive = mbar_wait(barrier(QUERY_FULL + warp / 4), 0, watchdog, STATUS_DENSE | 10);
-            alive = __all_sync(0xffffffffu, alive);
+            // shuffles and arithmetic, so a warp has ROWS_AT_ONCE of them under way, the angles of
+            // the next ones on their way meanwhile and the first ones' sines taken before the query
+            // is there. The places in shared memory are worked out once. Of a CTA of eight windows of 1,025
+            // tokens with 16 heads of 64 and 32 pairs it takes 9,000 of 39,000 cycles; with four rows
+            // at once, sincosf, whose branches keep rows from overlapping, and an address worked out
+            // for every access it took 20,000 of 49,000 (133.5 us the call, now 109.6).
             constexpr int PAIR_SLOTS = DIM / 64;  // pairs of a lane: 2 * pairs <= DIM
             constexpr int OTHER_SLOTS = DIM / 32; // dimensions behind the pairs
-            constexpr int ROWS_AT_ONCE = 4;
+            constexpr int ROWS_AT_ONCE = 8; // one turn of the swizzle
             constexpr int ROWS_OF_WARP = QUERY_TILES * TILE_M / SOFTMAX_WARPS;
             static_assert(ROWS_OF_WARP % ROWS_AT_ONCE == 0, "no rows are left over");
             const int others = DIM - 2 * rope.pairs;
-            // Where dimension `index` of query row `query_row` lies: 16-byte chunk c of a row sits
-            // at chunk c ^ (row % 8) of its 128-byte line.
-            auto address = [&](int query_row, int index) {
-                const int tile_row = query_row % TILE_M;
-                const int chunk = ((index % 64) / 8) ^ (tile_row % 8);
-                return base + SMEM_QUERY + (query_row / TILE_M) * TILE_BYTES +
-                       (index / 64) * SLAB_BYTES + tile_row * 128 + chunk * 16 + (index % 8) * 2;
+            // Where dimension `index` lies in a row whose number is a multiple of eight; 16-byte
+            // chunk c of the row `at` further on sits at chunk c ^ at of its 128-byte line.
+            auto place = [](int index) {
+                return static_cast<uint32_t>((index / 64) * SLAB_BYTES + (index % 64) * 2);
             };
-            auto load = [&](int query_row, int index) {
+            uint32_t first_places[PAIR_SLOTS], second_places[PAIR_SLOTS], other_places[OTHER_SLOTS];
+            bool paired[PAIR_SLOTS], unpaired[OTHER_SLOTS];
+            #pragma unroll
+            for (int slot = 0; slot < PAIR_SLOTS; slot++) {
+                const int pair = slot * 32 + lane;
+                paired[slot] = pair < rope.pairs;
+                first_places[slot] = place(pair);
+                second_places[slot] = place(paired[slot] ? pair + rope.pairs : 0);
+            }
+            #pragma unroll
+            for (int slot = 0; slot < OTHER_SLOTS; slot++) {
+                const int index = slot * 32 + lane;
+                unpaired[slot] = index < others;
+                other_places[slot] = place(unpaired[slot] ? 2 * rope.pairs + index : 0);
+            }
+            auto load = [](uint32_t rows, int at, uint32_t where) {
                 uint16_t bits;
-                asm volatile("ld.shared.u16 %0, [%1];" : "=h"(bits) : "r"(address(query_row, index)));
+                asm volatile("ld.shared.u16 %0, [%1];"
+                             : "=h"(bits)
+                             : "r"(rows + at * 128 + (where ^ (at << 4))));
                 return Element<HALF, DIM>::to_float(bits);
             };
-            auto store = [&](int query_row, int index, float value) {
+            auto store = [](uint32_t rows, int at, uint32_t where, float value) {
                 const uint16_t bits = Element<HALF, DIM>::from_float(value);
-                asm volatile("st.shared.u16 [%0], %1;" ::"r"(address(query_row, index)), "h"(bits)
+                asm volatile("st.shared.u16 [%0], %1;" ::"r"(rows + at * 128 + (where ^ (at << 4))),
+                             "h"(bits)
                              : "memory");
             };
+            float angles[ROWS_AT_ONCE][PAIR_SLOTS];
+            // Rows past the last token are zeroes; they are worked on and stored like the rest,
+            // with the last token's angles.
+            auto load_angles = [&](int first_row) {
+                #pragma unroll
+                for (int at = 0; at < ROWS_AT_ONCE; at++) {
+                    const int token = min(first_query + first_row + at, tokens - 1);
+                    const float *row = rope.angles + static_cast<int64_t>(token) * rope.pairs + lane;
+                    #pragma unroll
+                    for (int slot = 0; slot < PAIR_SLOTS; slot++) {
+                        angles[at][slot] = paired[slot] ? __ldg(row + slot * 32) : 0.0f;
+                    }
+                }
+            };
+            float2 turns[ROWS_AT_ONCE][PAIR_SLOTS]; // sine, cosine
+            auto take_turns = [&]() {
+                bool small = true;
+                #pragma unroll
+                for (int at = 0; at < ROWS_AT_ONCE; at++) {
+                    #pragma unroll
+                    for (int slot = 0; slot < PAIR_SLOTS; slot++) {
+                        small = small && fabsf(angles[at][slot]) <= ANGLE_LIMIT;
+                        turns[at][slot] = sine_and_cosine(angles[at][slot]);
+                    }
+                }
+                if (!__all_sync(0xffffffffu, small)) {
+                    #pragma unroll
+                    for (int at = 0; at < ROWS_AT_ONCE; at++) {
+                        #pragma unroll
+                        for (int slot = 0; slot < PAIR_SLOTS; slot++) {
+                            turns[at][slot] = sine_and_cosine_of_any(angles[at][slot]);
+                        }
+                    }
+                }
+            };
+            const int warp_begin = warp * ROWS_OF_WARP;
+            load_angles(warp_begin);
+            take_turns();
+            alive = mbar_wait(barrier(QUERY_FULL + warp / 4), 0, watchdog, STATUS_DENSE | 10);
+            alive = __all_sync(0xffffffffu, alive);
             const int rows_here = alive ? min(tokens - first_query, QUERY_TILES * TILE_M) : 0;
-            const int warp_end = min(rows_here, (warp + 1) * ROWS_OF_WARP);
+            const int warp_end = min(rows_here, warp_begin + ROWS_OF_WARP);
             #pragma unroll 1
-            for (int first_row = warp * ROWS_OF_WARP; first_row < warp_end;
-                 first_row += ROWS_AT_ONCE) {
-                // Rows past the last token are zeroes; they are worked on and stored like the rest,
-                // with the last token's angles.
-                float angle[ROWS_AT_ONCE][PAIR_SLOTS];
+            for (int first_row = warp_begin; first_row < warp_end; first_row += ROWS_AT_ONCE) {
+                load_angles(min(first_row + ROWS_AT_ONCE, warp_begin + ROWS_OF_WARP - 1));
+                const uint32_t rows = base + SMEM_QUERY + (first_row / TILE_M) * TILE_BYTES +
+                                      (first_row % TILE_M) * 128;
                 float first[ROWS_AT_ONCE][PAIR_SLOTS], second[ROWS_AT_ONCE][PAIR_SLOTS];
                 float other[ROWS_AT_ONCE][OTHER_SLOTS];
                 float squares[ROWS_AT_ONCE];
                 #pragma unroll
                 for (int at = 0; at < ROWS_AT_ONCE; at++) {
-                    const int token = min(first_query + first_row + at, tokens - 1);
-                    #pragma unroll
-                    for (int slot = 0; slot < PAIR_SLOTS; slot++) {
-                        const int pair = slot * 32 + lane;
-                        angle[at][slot] =
-                            pair < rope.pairs
-                                ? __ldg(rope.angles + static_cast<int64_t>(token) * rope.pairs + pair)
-                                : 0.0f;
-                    }
-                }
-                #pragma unroll
-                for (int at = 0; at < ROWS_AT_ONCE; at++) {
                     squares[at] = 0.0f;
                     #pragma unroll
                     for (int slot = 0; slot < PAIR_SLOTS; slot++) {
-                        const int pair = slot * 32 + lane;
-                        const bool here = pair < rope.pairs;
-                        first[at][slot] = here ? load(first_row + at, pair) : 0.0f;
-                        second[at][slot] = here ? load(first_row + at, pair + rope.pairs) : 0.0f;
+                        first[at][slot] = paired[slot] ? load(rows, at, first_places[slot]) : 0.0f;
+                        second[at][slot] = paired[slot] ? load(rows, at, second_places[slot]) : 0.0f;
                         squares[at] = fmaf(first[at][slot], first[at][slot], squares[at]);
                         squares[at] = fmaf(second[at][slot], second[at][slot], squares[at]);
                     }
                     #pragma unroll
                     for (int slot = 0; slot < OTHER_SLOTS; slot++) {
-                        const int index = slot * 32 + lane;
-                        other[at][slot] =
-                            index < others ? load(first_row + at, 2 * rope.pairs + index) : 0.0f;
+                        other[at][slot] = unpaired[slot] ? load(rows, at, other_places[slot]) : 0.0f;
                         squares[at] = fmaf(other[at][slot], other[at][slot], squares[at]);
                     }
                 }
@@ -466,24 +538,22 @@ __global__ void __launch_bounds__(THREADS, 1)
                     const float inverse = rsqrtf(squares[at] / DIM + rope.epsilon);
                     #pragma unroll
                     for (int slot = 0; slot < PAIR_SLOTS; slot++) {
-                        const int pair = slot * 32 + lane;
-                        if (pair < rope.pairs) {
-                            float sine, cosine;
-                            sincosf(angle[at][slot], &sine, &cosine);
+                        if (paired[slot]) {
+                            const float sine = turns[at][slot].x, cosine = turns[at][slot].y;
                             const float one = first[at][slot] * inverse;
                             const float two = second[at][slot] * inverse;
-                            store(first_row + at, pair, one * cosine - two * sine);
-                            store(first_row + at, pair + rope.pairs, one * sine + two * cosine);
+                            store(rows, at, first_places[slot], one * cosine - two * sine);
+                            store(rows, at, second_places[slot], one * sine + two * cosine);
                         }
                     }
                     #pragma unroll
                     for (int slot = 0; slot < OTHER_SLOTS; slot++) {
-                        const int index = slot * 32 + lane;
-                        if (index < others) {
-                            store(first_row + at, 2 * rope.pairs + index, other[at][slot] * inverse);
+                        if (unpaired[slot]) {
+                            store(rows, at, other_places[slot], other[at][slot] * inverse);
                         }
                     }
                 }
+                take_turns();
             }
             // The MMAs read the tiles through the async proxy.
             fence_proxy_async();

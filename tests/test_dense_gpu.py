@@ -358,10 +358,10 @@ def test_heads_of_64_and_the_fused_query_rope(reference_kernels, element_type, h
     (64, 1, 32), (64, 127, 20), (64, 129, 1), (64, 257, 31), (64, 518, 32),
     (128, 5, 64), (128, 131, 33), (128, 300, 40), (128, 255, 3),
 ])
-@pytest.mark.parametrize("element_type", [0, 1])
-def test_fused_query_rope_against_float64(element_type, head_dim, tokens, pairs):
+@pytest.mark.parametrize("element_type,span", [(0, 40.0), (1, 40.0), (1, 2e5)])
+def test_fused_query_rope_against_float64(element_type, span, head_dim, tokens, pairs):
     """Every split of a head into pairs and the rest, rows that fill a warp's turn and rows that do
-    not; the bound of the tests above."""
+    not, angles past what is reduced without a branch; the bound of the tests above."""
     heads, batch, epsilon = 3, 2, 1e-6
     scale = 1.0 / head_dim ** 0.5
     dtype = torch.float16 if element_type == 1 else torch.bfloat16
@@ -372,7 +372,7 @@ def test_fused_query_rope_against_float64(element_type, head_dim, tokens, pairs)
     inner = heads * head_dim
     layout = attention.make_layout((inner,) * 4, head_stride=(head_dim,) * 4,
                                    batch_stride=(tokens * inner,) * 4)
-    angles = torch.rand((tokens, pairs), generator=generator) * 80.0 - 40.0
+    angles = torch.rand((tokens, pairs), generator=generator) * (2 * span) - span
     ours = torch.zeros((batch, tokens, heads, head_dim), dtype=dtype, device="cuda")
     attention.attention_roped(element_type, head_dim, q.cuda(), k.cuda(), v.cuda(), ours, tokens,
                               heads, batch, layout, scale, angles.cuda(), pairs, epsilon)
