@@ -760,16 +760,26 @@ template <bool NORMALIZE, bool STATS, bool QUANTIZE>
 int launch(InputsParams params, int blocks, cudaStream_t stream) {
     const bool rotate = NORMALIZE && params.angles != nullptr && params.pairs > 0;
     // A CTA takes several heads, so that the sincosf of its block's angles are paid once and the next
-    // head's rows are in flight while one is worked on: as many as leave the grid a few CTAs for
-    // every place on the multiprocessors. (Without angles, the INT8/FP8 call on 16,896 raw tokens of
-    // 56 heads: 5,859 us with a head a CTA, 5,817 this way.)
-    const int wanted = 4 * 2 * max(multiprocessor_count(), 1);
-    params.heads_per_cta = HEADS_PER_CTA;
-    while (params.heads_per_cta > 1 &&
-           static_cast<int64_t>(blocks) *
-                   ((params.heads + params.heads_per_cta - 1) / params.heads_per_cta) <
-               wanted) {
-        params.heads_per_cta /= 2;
+    // head's rows are in flight while one is worked on. How many: the fewest that bring the rounds of
+    // the device times the length of a CTA within 3.5 % of the least, in units of half a turn (a
+    // head's q, k or v), of which a CTA's beginning takes one for the first rows to arrive, or four
+    // with the sincosf. Against powers of two with four rounds left, which it replaces: norm and RoPE of 1,101
+    // tokens and 56 heads 43.8 -> 35 us, the quantizer's two passes over 2,085 tokens and 56 heads
+    // 61 -> 56, the prepared INT8/FP8 inputs of 9,000 tokens and 32 heads 165 -> 155.
+    const int slots = ((NORMALIZE || QUANTIZE) ? 2 : 4) * max(multiprocessor_count(), 1);
+    const int turns = params.last_part - params.first_part + 1;
+    auto cost = [&](int heads_each) {
+        const int64_t ctas =
+            static_cast<int64_t>(blocks) * ((params.heads + heads_each - 1) / heads_each);
+        return (ctas + slots - 1) / slots * ((rotate ? 4 : 1) + 2 * turns * heads_each);
+    };
+    int64_t least = cost(1);
+    for (int heads_each = 2; heads_each <= HEADS_PER_CTA; heads_each++) {
+        least = min(least, cost(heads_each));
+    }
+    params.heads_per_cta = 1;
+    while (cost(params.heads_per_cta) * 1000 > least * 1035) {
+        params.heads_per_cta++;
     }
     if constexpr (NORMALIZE) {
         if (rotate && params.pairs % 16 == 0) {
