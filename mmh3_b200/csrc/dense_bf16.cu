@@ -230,6 +230,12 @@ __global__ void __launch_bounds__(THREADS, 1)
         CAUSAL ? static_cast<int>(gridDim.x) - 1 - linear / heads : static_cast<int>(blockIdx.x);
     const int item_of_batch = blockIdx.z;
     const int first_query = query_block * (QUERY_TILES * TILE_M);
+    // The last CTA of a sequence may have no row in its second tile. With heads of 64, where the two
+    // tiles share an exponential unit that is the bound, it is then left out (eight windows of 1,025
+    // tokens: 105.5 us with it, 102.6 without); with heads of 128 the question costs the long
+    // sequences more (57.9 ms and 58.3 at 66,048 tokens).
+    const bool second_tile = DIM != 64 || first_query + TILE_M < tokens;
+    const int last_tile = second_tile ? 1 : 0;
     // A causal row sees the keys up to its own token: the CTA's two query tiles need the key
     // blocks up to the second tile's diagonal one (the first tile finds its last block all masked).
     const int blocks = CAUSAL ? min((tokens + TILE_N - 1) / TILE_N,
@@ -346,7 +352,9 @@ __global__ void __launch_bounds__(THREADS, 1)
             }
             if (alive) {
                 tcgen05_fence_after();
-                score(1, ring);
+                if (second_tile) {
+                    score(1, ring);
+                }
                 tcgen05_commit(barrier(RING_EMPTY + 0));
             }
             int item = 1; // ring position of V of the current block; K of the next follows it
@@ -366,6 +374,9 @@ __global__ void __launch_bounds__(THREADS, 1)
                 const uint32_t key_tile = ring + key_stage * TILE_BYTES;
                 #pragma unroll
                 for (int tile = 0; tile < QUERY_TILES; tile++) {
+                    if (tile > last_tile) {
+                        break;
+                    }
                     // The first 64 keys' probabilities are handed over first: their four MMAs
                     // run while the softmax threads work on the other 64, which takes a quarter
                     // of O += P V out of the chain softmax -> P V -> S of a tile (62.4 -> 60.8 ms).
@@ -383,13 +394,13 @@ __global__ void __launch_bounds__(THREADS, 1)
                     }
                     tcgen05_fence_after();
                     accumulate(tile, value_tile, false, TILE_N / 32, TILE_N / 16);
-                    if (tile == QUERY_TILES - 1) {
+                    if (tile == last_tile) {
                         tcgen05_commit(barrier(RING_EMPTY + value_stage));
                     }
                     if (more) {
                         // Issued after the P V that reads the columns it overwrites.
                         score(tile, key_tile);
-                        if (tile == QUERY_TILES - 1) {
+                        if (tile == last_tile) {
                             tcgen05_commit(barrier(RING_EMPTY + key_stage));
                         }
                     }
@@ -559,6 +570,7 @@ __global__ void __launch_bounds__(THREADS, 1)
             fence_proxy_async();
             mbar_arrive(barrier(QUERY_READY));
         }
+        alive = alive && tile <= last_tile;
         for (int block = 0; alive && block < blocks; block++) {
             alive = mbar_wait(barrier(SCORES_FULL + tile), block & 1, watchdog, STATUS_DENSE | 7);
             // The tensor memory accesses below are warp-wide: the warp goes on or leaves as one.
