@@ -121,13 +121,13 @@ template <bool HALF, int DIM = 128> struct Element {
 constexpr float RESCALE_THRESHOLD = 8.0f;
 // Of every eight pairs of probabilities, how many take the polynomial exp2 instead of the MUFU. With
 // heads of 64 the MMAs are half as long and the exponentials bound a block: eight windows of 1,025
-// tokens with 16 heads take 137.2 us with none, 131.9 with two, 131.3 with three and 142.5 with four
-// (the FMA pipe is then the fuller one); looking for NaNs, which the polynomial has none of, makes
-// 133.5 of three. The error against 64 bits stays at 3.58e-4 (FP16). With
-// heads of 128 two of eight cost fewer cycles a block (3,466 against 3,543) and more power: over
-// the twenty launches of a benchmark run the GPU sits at its power cap, where none runs at 1,627
-// MHz instead of 1,582 and is the faster by 0.6 % (2 % in the token attention over routes).
-template <int DIM> constexpr int POLYNOMIAL_PAIRS_OF_8 = DIM == 64 ? 3 : 0;
+// tokens with 16 heads take 108.3 us with none, 105.4 with two and 109.8 with three (the FMA pipe is
+// then the fuller one). A polynomial of degree five would make 104.3 of two, one of degree four 102.5
+// of three, but they are further from 2^x than the MUFU is. With heads of 128 the MUFU takes them
+// all: a cubic for one pair in four cost fewer cycles a block (3,466 against 3,543) and more power, and
+// over the twenty launches of a benchmark run the GPU sits at its power cap, where none ran at 1,627
+// MHz instead of 1,582 and was the faster by 0.6 % (2 % in the token attention over routes).
+template <int DIM> constexpr int POLYNOMIAL_PAIRS_OF_8 = DIM == 64 ? 2 : 0;
 
 struct DenseMaps {
     CUtensorMap query;

@@ -246,3 +246,22 @@ extern "C" int mmh3_b200_expired_wait_selftest(unsigned int code) {
     cudaFree(gave_up);
     return error == cudaSuccess ? count : -static_cast<int>(error);
 }
+
+namespace {
+
+__global__ void exp2_kernel(const float2 *__restrict__ in, float2 *__restrict__ out, int pairs) {
+    const int index = blockIdx.x * blockDim.x + threadIdx.x;
+    if (index < pairs) {
+        out[index] = sm100::exp2_polynomial(in[index]);
+    }
+}
+
+} // namespace
+
+// 2^x of `pairs` pairs of floats as the attention's polynomial gives it. Device memory, 8-byte
+// aligned; returns a cudaError_t.
+extern "C" int mmh3_b200_exp2_selftest(const void *in, void *out, int pairs) {
+    exp2_kernel<<<(pairs + 255) / 256, 256>>>(static_cast<const float2 *>(in),
+                                              static_cast<float2 *>(out), pairs);
+    return static_cast<int>(cudaGetLastError());
+}

@@ -385,7 +385,7 @@ def test_fused_query_rope_against_float64(element_type, span, head_dim, tokens, 
 
 @pytest.mark.parametrize("element_type", [0, 1])
 def test_heads_of_64_whose_exponentials_come_two_ways(element_type):
-    """Three of eight pairs of keys take a polynomial: every key alone in turn holds a row's weight or a
+    """Two of eight pairs of keys take a polynomial: every key alone in turn holds a row's weight or a
     NaN, and scores far below the maximum weigh nothing."""
     tokens, heads, head_dim = 128, 2, 64
     dtype = torch.float16 if element_type == 1 else torch.bfloat16
@@ -413,6 +413,60 @@ def test_heads_of_64_whose_exponentials_come_two_ways(element_type):
         poisoned[column, 0, 0] = float("nan")
         result = run(poisoned)
         assert torch.isnan(result[:, 0]).all() and torch.isfinite(result[:, 1]).all()
+
+
+def test_the_polynomial_exponential_is_as_close_as_the_unit_it_relieves():
+    """exp2_polynomial against float64. Its fit is off by 2.0e-9, the rounding of its coefficients by
+    1e-8; the last FMA rounds by half a unit of a result of 0.707 to 1.415 (6.0e-8 of it at most), the
+    one before by half a unit of a number under one, times a fraction of a half over the result (2.1e-8),
+    and the others by less: 1.1e-7 in all. ex2.approx is within 1.45e-7."""
+    library = load_selftest()
+    count = 1 << 22
+    generator = torch.Generator().manual_seed(5)
+    x = torch.rand(count, generator=generator, dtype=torch.float64) * 133.0 - 125.0
+    # Near the whole numbers and half-way between them, where n changes.
+    x[:4096] = torch.arange(4096).double() / 32.0 - 120.0
+    x[4096:8192] = x[:4096] * (1.0 + 2.0 ** -23)
+    x = x.float().cuda()
+
+    def evaluate(values):
+        result = torch.empty_like(values)
+        assert library.mmh3_b200_exp2_selftest(
+            ctypes.c_void_p(values.data_ptr()), ctypes.c_void_p(result.data_ptr()),
+            values.numel() // 2) == 0
+        torch.cuda.synchronize()
+        return result
+
+    exact = torch.exp2(x.double())
+    assert float(((evaluate(x).double() - exact) / exact).abs().max()) <= 1.1e-7
+    # Nothing is left of what the MUFU gives zero for, but for denormals above -127.
+    low = torch.tensor([-127.0, -127.5, -1e4, -3e38, float("-inf"), float("nan")], device="cuda")
+    assert torch.equal(evaluate(low).view(torch.int32), torch.zeros(6, dtype=torch.int32).cuda())
+    between = torch.linspace(-126.999, -125.0, 1000, device="cuda")
+    values = evaluate(between).double()
+    assert (values >= 0).all() and (values <= torch.exp2(between.double()) * (1 + 1.1e-7)).all()
+
+
+@pytest.mark.parametrize("tokens", [1, 63, 64, 130, 300])
+def test_later_values_do_not_reach_causal_rows_of_heads_of_64(tokens):
+    """A masked key weighs exactly nothing in BF16, whose smallest numbers times the largest values
+    are not small: rows are the same bits whatever finite values the tokens after them have."""
+    heads, head_dim, later = 2, 64, 300
+    layout = attention.make_layout((heads * head_dim,) * 4, head_stride=(head_dim,) * 4, causal=1)
+    generator = torch.Generator().manual_seed(tokens)
+    q, k, v = (torch.randn((tokens + later, heads, head_dim), generator=generator).bfloat16().cuda()
+               for _ in range(3))
+
+    def run(values):
+        output = torch.zeros_like(q)
+        attention.attention(0, head_dim, q, k, values, output, tokens + later, heads, 1, layout,
+                            0.125)
+        assert attention.take_status() == 0
+        return output[:tokens].view(torch.int16)
+
+    huge = v.clone()
+    huge[tokens:] = 3e38
+    assert torch.equal(run(huge), run(v))
 
 
 def test_unsupported_combinations_report_an_error():
