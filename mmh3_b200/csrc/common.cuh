@@ -73,9 +73,10 @@ struct SharedMemoryOptIn {
     }
 };
 
-// Launches a kernel that begins with let_next_kernel_begin and waits with wait_for_kernels_before
-// (sm100.cuh) before it reads or writes global memory: its launch, and the set-up of its CTAs on
-// multiprocessors that the kernel before it has left, then overlap the end of that kernel. It is
+// Launches a kernel that waits with wait_for_kernels_before (sm100.cuh) before it reads or writes
+// global memory or takes tensor memory, and calls let_next_kernel_begin once it has its tensor memory
+// (at its beginning, if it takes none): its launch, and the set-up of its CTAs on multiprocessors
+// that the kernel before it has left, then overlap the end of that kernel. It is
 // for the kernels that short calls are made of: INT8/FP8 attention of 2,085 tokens and 56 heads (four
 // kernels) went from 213 us to 204, a causal prompt of 300 tokens (one, behind its like) from 13.0
 // to 12.0. Those of VSA and Sol-Attn, whose calls take milliseconds, are launched as ever.

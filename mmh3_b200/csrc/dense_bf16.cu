@@ -216,7 +216,6 @@ __global__ void __launch_bounds__(THREADS, 1)
     const Watchdog watchdog = {abort_flag, status};
     auto barrier = [&](int index) { return barriers + index * 8; };
 
-    let_next_kernel_begin();
     const int warp = warp_index();
     const int lane = threadIdx.x % 32;
     // Causal CTAs cost what their place in the sequence does: the most expensive ones of all heads
@@ -259,13 +258,14 @@ __global__ void __launch_bounds__(THREADS, 1)
         fence_barrier_init();
         fence_proxy_async();
     }
+    wait_for_kernels_before();
     if (warp == MMA_WARP) {
         tmem_alloc(smem_u32(const_cast<uint32_t *>(tmem_slot)), TMEM_COLUMNS);
     }
-    wait_for_kernels_before();
     tcgen05_fence_before();
     // Once a wait has run out anywhere, the rest of the grid drains instead of waiting too.
     const bool stopped = __syncthreads_or(*reinterpret_cast<volatile unsigned int *>(status) != 0);
+    let_next_kernel_begin();
     tcgen05_fence_after();
     const uint32_t tmem = *tmem_slot;
     if (stopped) {

@@ -174,7 +174,6 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1)
     volatile uint32_t *tmem_slot = &tmem_slot_storage;
     const Watchdog watchdog{abort_flag, status};
     auto barrier = [&](int index) { return smem_u32(&barriers[index]); };
-    let_next_kernel_begin();
     const int warp = warp_index();
     const int lane = threadIdx.x % 32;
     const int tiles = walk.tiles();
@@ -203,6 +202,7 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1)
         fence_barrier_init();
         fence_proxy_async();
     }
+    wait_for_kernels_before();
     if (warp == MMA_WARP) {
         if constexpr (PAIR) {
             tmem_alloc_pair(smem_u32(const_cast<uint32_t *>(tmem_slot)), TMEM_COLUMNS);
@@ -215,7 +215,7 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1)
     if constexpr (PAIR) {
         cluster_sync();
     }
-    wait_for_kernels_before();
+    let_next_kernel_begin();
     tcgen05_fence_after();
     const uint32_t tmem = *tmem_slot;
 

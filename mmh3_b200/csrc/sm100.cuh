@@ -45,9 +45,14 @@ __device__ __forceinline__ bool elect_one() {
 
 // ---------------------------------------------------------------------------------------------
 // Kernels launched with launch_behind (common.cuh): the next kernel of the stream may be set up
-// once every CTA of this one has begun, and waits here for the kernels before it to have finished
+// once every CTA of this one has said so, and waits here for the kernels before it to have finished
 // and their writes to be visible, before it touches global memory. Every thread waits, so no kernel
 // ends before the ones it was launched behind.
+//
+// Tensor memory is what CTAs of two kernels on one multiprocessor could wait for each other over: one
+// that holds it and waits for the kernel before, one of that kernel that waits in its tcgen05.alloc,
+// where no limit ends the wait. So a kernel takes its columns after wait_for_kernels_before, and lets
+// the next one begin when it has them, whatever fits beside what.
 
 __device__ __forceinline__ void let_next_kernel_begin() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
