@@ -258,7 +258,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         fence_barrier_init();
         fence_proxy_async();
     }
-    wait_for_kernels_before();
+    [[maybe_unused]] const int behind = wait_for_kernels_before();
     if (warp == MMA_WARP) {
         tmem_alloc(smem_u32(const_cast<uint32_t *>(tmem_slot)), TMEM_COLUMNS);
     }
@@ -478,7 +478,8 @@ __global__ void __launch_bounds__(THREADS, 1)
                 #pragma unroll
                 for (int at = 0; at < ROWS_AT_ONCE; at++) {
                     const int token = min(first_query + first_row + at, tokens - 1);
-                    const float *row = rope.angles + static_cast<int64_t>(token) * rope.pairs + lane;
+                    const float *row = rope.angles + static_cast<int64_t>(token) * rope.pairs + lane +
+                                       behind;
                     #pragma unroll
                     for (int slot = 0; slot < PAIR_SLOTS; slot++) {
                         angles[at][slot] = paired[slot] ? __ldg(row + slot * 32) : 0.0f;

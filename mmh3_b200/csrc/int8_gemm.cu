@@ -202,7 +202,7 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1)
         fence_barrier_init();
         fence_proxy_async();
     }
-    wait_for_kernels_before();
+    const int behind = wait_for_kernels_before();
     if (warp == MMA_WARP) {
         if constexpr (PAIR) {
             tmem_alloc_pair(smem_u32(const_cast<uint32_t *>(tmem_slot)), TMEM_COLUMNS);
@@ -348,7 +348,8 @@ __global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1)
                            epilogue_warp * STAGING_BYTES;
         int round = 0;
         bool alive = true;
-        for (int tile = first_tile; alive && tile < tiles; tile += tile_step, round++) {
+        // The scales and the bias are read at places that follow from `behind`.
+        for (int tile = first_tile + behind; alive && tile < tiles; tile += tile_step, round++) {
             const int buffer = round % ACCUMULATORS;
             int tile_m, tile_n;
             walk.locate(tile, tile_m, tile_n);

@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         fence_barrier_init();
         fence_proxy_async();
     }
-    wait_for_kernels_before();
+    const int behind = wait_for_kernels_before();
     if (warp == MMA_WARP) {
         tmem_alloc(smem_u32(const_cast<uint32_t *>(tmem_slot)), TMEM_COLUMNS);
     }
@@ -292,11 +292,11 @@ __global__ void __launch_bounds__(THREADS, 1)
         const uint32_t lane_base = static_cast<uint32_t>((warp % 4) * 32) << 16;
         const uint32_t scores = tmem + lane_base + TMEM_SCORES + tile * TILE_N;
         const uint32_t accumulator = tmem + lane_base + TMEM_OUTPUT + tile * HEAD_DIM;
-        const float *head_key_scales = key_scales + static_cast<size_t>(head) * blocks64;
+        const float *head_key_scales = key_scales + static_cast<size_t>(head) * blocks64 + behind;
         // Rows past the last token read no scale; their scores are zero and never stored.
         const float query_factor =
             scale_log2 * (token < tokens ? query_scales[static_cast<size_t>(head) * blocks64 +
-                                                        token / 64]
+                                                        token / 64 + behind]
                                          : 0.0f);
         float maximum = -FLT_MAX;
         float2 sums[2] = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};
@@ -452,7 +452,7 @@ __global__ void __launch_bounds__(THREADS, 1)
             tcgen05_fence_after();
             // The sums carry the factor of 448 the probabilities do.
             const float inverse =
-                value_scales[head] / ((sums[0].x + sums[0].y) + (sums[1].x + sums[1].y));
+                value_scales[head + behind] / ((sums[0].x + sums[0].y) + (sums[1].x + sums[1].y));
             __nv_bfloat16 *output_row =
                 output + static_cast<int64_t>(token) * output_token_stride +
                 static_cast<int64_t>(head) * output_head_stride;

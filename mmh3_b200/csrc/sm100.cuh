@@ -58,9 +58,10 @@ __device__ __forceinline__ void let_next_kernel_begin() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
-// Returns zero, for an address that a read-only load is to take only after the wait: such loads are
-// not held back by the clobber of memory.
-__device__ __forceinline__ int wait_for_kernels_before() {
+// Returns zero, for the addresses of read-only loads (__ldg, and what the compiler makes one of behind
+// a const __restrict__ pointer): the clobber of memory does not hold those back, and what the kernels
+// before have written is to be read after the wait.
+[[nodiscard]] __device__ __forceinline__ int wait_for_kernels_before() {
     int zero;
     asm volatile("griddepcontrol.wait;\n"
                  "mov.u32 %0, 0;"

@@ -52,3 +52,28 @@ def test_tensor_memory_changes_hands_without_a_circle(name, body):
     last = body.rindex("tmem_alloc")
     barrier = body.index("__syncthreads", last)
     assert wait < first <= last < barrier < begin
+
+
+# What each kernel reads through the read-only path of what a kernel before it may have written.
+READ_ONLY = {
+    "dense_bf16_kernel": {"rope.angles": "behind"},
+    "quantized_dense_kernel": {"query_scales[": "behind", "= key_scales +": "behind",
+                               "value_scales[": "behind"},
+    # Rows and columns follow from the tile, which follows from the wait.
+    "int8_gemm_kernel": {"tile = first_tile +": "behind"},
+    "inputs_kernel": {"block = blockIdx.x +": "wait_for_kernels_before()"},
+    "value_scales_kernel": {"block = threadIdx.x +": "wait_for_kernels_before()"},
+}
+
+
+@pytest.mark.parametrize("name,body", behind(), ids=lambda value: value if "{" not in value else "")
+def test_read_only_loads_follow_from_the_wait(name, body):
+    """A read-only load may be moved before an asm statement that clobbers memory, but not before the
+    value its address is made of: the zero that the wait returns is in each of them."""
+    assert not re.search(r"[;{}]\s*wait_for_kernels_before\(\);", body)
+    for begin, token in READ_ONLY[name].items():
+        places = [match.start() for match in re.finditer(re.escape(begin), body)]
+        assert places, begin
+        for place in places:
+            statement = body[place:body.index(";", place)]
+            assert token in statement, statement
