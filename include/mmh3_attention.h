@@ -86,7 +86,8 @@ typedef struct Mmh3VsaWorkspace {
  * VAE decoder's uses. `scale` must be positive. Operands TMA cannot describe (bases or strides that
  * are not multiples of 16 bytes) are first gathered into dense arrays in stream-ordered scratch
  * (cudaMallocAsync on `stream`, given back with cudaFreeAsync behind the kernel); the result is
- * the same bits.
+ * the same bits. The output may take the query's place, element by element. An item's output may lie
+ * over other items' operands or outputs: the items are then worked on in their order.
  * Replaces crates/mmh3-cuda/kernels/attention.cu:531-536. */
 int mmh3_attention(int element_type, int head_dim, const void *query, const void *key,
                    const void *value, void *output, int tokens, int heads, int batch,

@@ -23,8 +23,8 @@
 // Tensor memory: S0 | S1 | O0 | O1, S 128 columns each and O one column per head dimension.
 #include <cfloat>
 #include <cmath>
-#include <utility>
 
+#include "batch_items.cuh"
 #include "common.cuh"
 #include "sm100.cuh"
 
@@ -769,41 +769,19 @@ bool encode_operand(CUtensorMap *map, bool half, int head_dim, const void *base,
         dimensions, strides, box);
 }
 
-// Whether no two items of the output share an element, whatever the order of its dimensions: taken
-// from the smallest stride up, each dimension steps over all that the ones before it span.
-bool output_items_disjoint(int tokens, int heads, int head_dim, int batch,
-                           const Mmh3AttentionLayout &layout) {
-    int64_t strides[3] = {layout.token_stride[OUTPUT], layout.head_stride[OUTPUT],
-                          layout.batch_stride[OUTPUT]};
-    int64_t sizes[3] = {tokens, heads, batch};
-    int64_t span = head_dim;
-    for (int taken = 0; taken < 3; taken++) {
-        int next = taken;
-        for (int index = taken + 1; index < 3; index++) {
-            next = strides[index] < strides[next] ? index : next;
-        }
-        std::swap(strides[taken], strides[next]);
-        std::swap(sizes[taken], sizes[next]);
-        if (sizes[taken] > 1 && strides[taken] < span) {
-            return false;
-        }
-        span += strides[taken] * (sizes[taken] - 1);
-    }
-    return true;
-}
-
 // Whether every item of a batch can go in one launch: TMA can describe the three operands as they
 // are, batches included, and the grid holds them. A batch of items smaller than the device then
 // fills it instead of leaving most of it idle once per item: eight windows of 1,025 tokens with 16
 // heads of 64 are 80 CTAs an item on 148 SMs, 348 us item by item and 180 in one launch.
 // What stays with a launch per item: operands off TMA's 16-byte grid, whose copies are made item
 // by item so that the scratch is one item's, batch strides TMA cannot hold (zero, negative or
-// of 2^40 bytes and more), and items whose outputs overlap, which are written in order.
-bool batch_in_one_launch(const uint16_t *const (&bases)[3], int tokens, int heads, int group,
+// of 2^40 bytes and more), and items whose outputs lie over other items' outputs or operands, which
+// are worked on in order.
+bool batch_in_one_launch(const void *const (&bases)[4], int tokens, int heads, int group,
                          int head_dim, int batch, const Mmh3AttentionLayout &layout) {
     constexpr int64_t STRIDE_LIMIT = int64_t{1} << 39; // in elements of two bytes
     constexpr int MOST_ITEMS = 65535;                  // of the grid's third dimension
-    if (batch > MOST_ITEMS || !output_items_disjoint(tokens, heads, head_dim, batch, layout)) {
+    if (batch > MOST_ITEMS) {
         return false;
     }
     for (int operand = 0; operand < 3; operand++) {
@@ -814,7 +792,7 @@ bool batch_in_one_launch(const uint16_t *const (&bases)[3], int tokens, int head
             return false;
         }
     }
-    return true;
+    return items_are_independent(bases, tokens, heads, group, head_dim, batch, layout);
 }
 
 // The kernel instance for an element type, mask, head dimension and query transform, and its
@@ -876,7 +854,7 @@ int launch_dense_bf16(const void *query, const void *key, const void *value, voi
     const auto *k = static_cast<const uint16_t *>(key);
     const auto *v = static_cast<const uint16_t *>(value);
     auto *out = static_cast<uint16_t *>(output);
-    const uint16_t *const whole[3] = {q, k, v};
+    const void *const whole[4] = {q, k, v, out};
     const int items = batch > 1 && batch_in_one_launch(whole, tokens, heads, group, head_dim, batch, layout)
                           ? batch
                           : 1;

@@ -8,6 +8,7 @@
 // mode 0: BF16 operands, FP32 accumulators, V [keys][dims] MN-major (kind::f16)
 // mode 1: INT8 A and B with INT32 accumulators (kind::i8); E4M3 P and V^T [dims][keys] K-major with
 //         FP32 accumulators (kind::f8f6f4)
+#include "../../mmh3_b200/csrc/batch_items.cuh"
 #include "../../mmh3_b200/csrc/common.cuh"
 #include "../../mmh3_b200/csrc/sm100.cuh"
 
@@ -264,4 +265,14 @@ extern "C" int mmh3_b200_exp2_selftest(const void *in, void *out, int pairs) {
     exp2_kernel<<<(pairs + 255) / 256, 256>>>(static_cast<const float2 *>(in),
                                               static_cast<float2 *>(out), pairs);
     return static_cast<int>(cudaGetLastError());
+}
+
+// The rule by which a batch of dense attention goes in one launch, over addresses that are never
+// read: 1 or 0.
+extern "C" int mmh3_b200_batch_items_selftest(const void *query, const void *key, const void *value,
+                                              const void *output, int tokens, int heads, int group,
+                                              int head_dim, int batch,
+                                              const Mmh3AttentionLayout *layout) {
+    return mmh3::items_are_independent({query, key, value, output}, tokens, heads, group, head_dim,
+                                       batch, *layout);
 }

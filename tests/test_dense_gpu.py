@@ -244,6 +244,29 @@ def test_a_batch_equals_its_items(element_type, head_dim, tokens, batch, causal,
     assert torch.equal(run(True).view(torch.int16), run(False).view(torch.int16))
 
 
+@pytest.mark.parametrize("operand,shift", [(0, -1), (0, 0), (0, 1), (1, -1), (1, 1), (2, -1), (2, 1)])
+def test_a_batch_whose_output_lies_over_its_operands(operand, shift):
+    """Item i's output over the query, keys or values of item i - 1 or i + 1, or in its own query's
+    place: the bits of one call per item, in order."""
+    tokens, heads, batch, head_dim = 700, 4, 3, 64
+    size = tokens * heads * head_dim
+    layout = attention.make_layout((heads * head_dim,) * 4, head_stride=(head_dim,) * 4,
+                                   batch_stride=(size,) * 4)
+    generator = torch.Generator().manual_seed(operand)
+    source = torch.randn((3, batch + 2, size), generator=generator).bfloat16().cuda()
+
+    def run(whole):
+        buffers = source.clone()
+        for item in range(1 if whole else batch):
+            views = [buffers[index, 1 + item:] for index in range(3)]
+            attention.attention(0, head_dim, *views, buffers[operand, 1 + item + shift:], tokens,
+                                heads, batch if whole else 1, layout, 0.125)
+        assert attention.take_status() == 0
+        return buffers
+
+    assert torch.equal(run(True).view(torch.int16), run(False).view(torch.int16))
+
+
 def reference_attention(q, k, v, group, causal):
     """softmax(q k^T * scale) v in float64 with torch, [batch, tokens, heads, 128] operands."""
     keys = k.double().repeat_interleave(group, dim=2)
