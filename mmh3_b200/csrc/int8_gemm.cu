@@ -773,7 +773,7 @@ int launch_int8_gemm(int config, int group_m, const int8_t *activations, const i
     if (output_stride <= 0) {
         output_stride = swiglu ? n / 2 : n;
     }
-    // The epilogue stores 16 bytes at a time (8 with SwiGLU) and reads the scales in pairs.
+    // The epilogue stores 16 bytes at a time and reads the scales in pairs.
     if (reinterpret_cast<uintptr_t>(output) % 16 != 0 || output_stride % 8 != 0 ||
         reinterpret_cast<uintptr_t>(weight_scales) % 8 != 0 ||
         reinterpret_cast<uintptr_t>(bias) % 8 != 0) {

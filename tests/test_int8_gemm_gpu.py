@@ -77,7 +77,7 @@ def run_reference(library, case, m, n, k, f16=False, swiglu=False, first_column=
 
 @pytest.mark.parametrize("m,n,k,f16,seed", [
     (300, 512, 384, False, 7),      # int8_gemm.rs:231-233
-    (2000, 3072, 384, False, 8),    # 236-240: more tiles than SMs, a ragged last row of tiles
+    (2000, 3072, 384, False, 8),    # 236-240: more tiles than pairs of CTAs, a ragged last row of them
     (600, 3072, 256, True, 11),     # 256-258: FP16 with a bias
     (257, 384, 128, False, 3),      # one row into the second tile, a last tile of 128 columns
 ])
@@ -143,6 +143,49 @@ def test_tiles_of_pairs_and_of_single_ctas_with_an_adapter(m, n, k, rank):
     assert np.array_equal(maxima, gemm_cases.column_maxima(bits, 0))
 
 
+@pytest.mark.parametrize("m,n", [
+    (100, 28672),  # single CTAs, a tile each
+    (300, 25088),  # single CTAs, most of them a second tile
+    (700, 28672),  # pairs, four or five tiles each
+])
+@pytest.mark.parametrize("rank", [0, 64])
+@pytest.mark.parametrize("f16", [False, True])
+@pytest.mark.parametrize("swiglu", [False, True])
+def test_every_instance_on_pairs_and_on_single_ctas(swiglu, f16, rank, m, n):
+    """Every epilogue (SwiGLU or not, BF16 or FP16, with an adapter or not, with a bias) in both forms
+    and over more than one tile, against the definition within the reference's bounds."""
+    k = 256
+    case = gemm_cases.operands(m, n, k, m + 2 * swiglu + f16, bias=True, swiglu=swiglu)
+    adapter = None
+    if rank:
+        adapter = (*gemm_cases.adapter_operands(m, n, rank, rank, 3, span=0.5), rank, 0.75)
+    products = gemm_cases.definition(*case, adapter=adapter)
+    if not swiglu:
+        bits, _ = run(case, m, n, k, f16=f16, adapter=adapter)
+        actual = gemm_cases.widen(bits, f16)
+        assert np.all(np.abs(actual - products) <= np.abs(products) / 256.0 + 1e-4)  # rs:212
+        return
+    a, w, a_scales, w_scales, bias = case
+    case = (a, gemm_cases.interleave(w), a_scales, gemm_cases.interleave(w_scales),
+            gemm_cases.interleave(bias))
+    if rank:
+        down, up, _, scale = adapter
+        adapter = (down, gemm_cases.interleave(up), rank, scale)
+    bits, _ = run(case, m, n, k, f16=f16, swiglu=True, adapter=adapter)
+    rounded = products.astype(np.float32)
+    if f16:
+        rounded = rounded.astype(np.float16).astype(np.float64)
+    else:
+        rounded = synthetic.bf16_bits_to_f32(synthetic.to_bf16_bits(rounded)).reshape(m, n)
+        rounded = rounded.astype(np.float64)
+    gate, up_values = rounded[:, :n // 2], rounded[:, n // 2:]
+    expected = gate / (1.0 + np.exp(-gate)) * up_values
+    # The bounds of test_swiglu_with_an_adapter: products that round the other way may leave the
+    # reference's bound, one in a hundred thousand, by little.
+    excess = np.abs(gemm_cases.widen(bits, f16) - expected) - (np.abs(expected) / 64.0 + 1e-3)
+    assert np.count_nonzero(excess > 0) <= 1e-5 * excess.size and excess.max() < 0.01
+
+
 @pytest.mark.parametrize("f16", [False, True])
 def test_swiglu_of_interleaved_rows(oracle, reference_kernels, f16):
     # int8_gemm.rs:269-383 without the adapter; the rows interleaved by the library itself.
@@ -177,7 +220,7 @@ def test_swiglu_of_interleaved_rows(oracle, reference_kernels, f16):
 
 @pytest.mark.parametrize("m,n,k,rank,stride,seed", [
     (300, 512, 256, 128, 128, 9),    # int8_gemm.rs:243-247
-    (600, 3072, 256, 384, 384, 10),  # the rank of the fused qkv adapters, more tiles than SMs
+    (600, 3072, 256, 384, 384, 10),  # the rank of the fused qkv adapters, a ragged last row of tiles
     (300, 512, 256, 64, 128, 12),    # 250-253: down rows wider than the rank
 ])
 def test_adds_a_low_rank_adapter(reference_kernels, m, n, k, rank, stride, seed):
