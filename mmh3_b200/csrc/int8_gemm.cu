@@ -706,11 +706,13 @@ int launch_tiles(const GemmTask &task, int in_flight, cudaStream_t stream) {
 // Tiles of 256 rows on pairs of CTAs, or of 128 on single ones where those need few enough rounds of
 // the device. A round is the same MMAs either way, but a single CTA takes 96 bytes a cycle from L2
 // instead of 64 (and with an adapter keeps eight epilogue warps): where both need the same number of
-// rounds pairs are the faster by up to a fifth, and at four rounds to five they are level. Pairs
-// and singles, m x n x k: 800 x 5,376 x 7,168 with an adapter (2 rounds and 1) 43.3 and 27.0 us, 300
-// x 12,288 x 4,096 (2 and 1) 26.2 and 17.6, 600 x 28,672 x 5,376 (5 and 4) 86.2 and 85.8, with an
-// adapter 105.4 and 108.6, 2,000 x 12,288 x 4,096 (6 and 6) 70.8 and 82.8, 1,300 x 21,504 x 7,168 with
-// an adapter (7 and 7) 158.5 and 187.2.
+// rounds pairs are the faster by up to a fifth, and at four rounds to five they are level, but with an
+// adapter and no SwiGLU singles are ahead by 3 %. Pairs and singles, m x n x k: 800 x 5,376 x 7,168 with
+// an adapter (2 rounds and 1) 43.3 and 27.0 us, 300 x 12,288 x 4,096 (2 and 1) 26.2 and 17.6; 600 x
+// 28,672 x 5,376 (5 and 4) 95.3 and 94.8, with SwiGLU 102.5 and 101.2, with an adapter of rank 64 106.6
+// and 102.9, with one of 384 117.4 and 113.4, with SwiGLU and rank 64 (640 rows) 107.4 and 109.0; 1,600 x
+// 14,336 x 5,376 with an adapter (6 and 5) 120.6 and 127.1; 2,000 x 12,288 x 4,096 (6 and 6) 70.8 and
+// 82.8, 1,300 x 21,504 x 7,168 with an adapter (7 and 7) 158.5 and 187.2.
 template <typename Output, bool SWIGLU, bool ADAPTED>
 int launch_kernel(const GemmTask &task, cudaStream_t stream) {
     const int processors = multiprocessor_count();
@@ -723,7 +725,8 @@ int launch_kernel(const GemmTask &task, cudaStream_t stream) {
         return ((task.m + static_cast<int64_t>(rows) - 1) / rows * columns + in_flight - 1) / in_flight;
     };
     const int64_t of_pairs = rounds(2 * TILE_M, pairs), of_singles = rounds(TILE_M, processors);
-    if (of_singles * 5 < of_pairs * 4) {
+    const int64_t singles = of_singles * 5, pairs_allow = of_pairs * 4;
+    if (ADAPTED && !SWIGLU ? singles <= pairs_allow : singles < pairs_allow) {
         return launch_tiles<Output, SWIGLU, ADAPTED, false>(task, processors, stream);
     }
     return launch_tiles<Output, SWIGLU, ADAPTED, true>(task, pairs, stream);

@@ -130,6 +130,7 @@ def test_tiles_of_pairs_and_of_single_ctas(oracle, m, n, k):
 @pytest.mark.parametrize("m,n,k,rank", [
     (1, 128, 128, 64), (129, 384, 640, 128), (700, 13312, 256, 64), (512, 28672, 384, 384),
     (513, 13312, 256, 64), (300, 28672, 384, 384),  # on single CTAs
+    (600, 28672, 128, 64),  # four rounds of single CTAs for five of pairs
 ])
 def test_tiles_of_pairs_and_of_single_ctas_with_an_adapter(m, n, k, rank):
     # The bounds of test_adds_a_low_rank_adapter.
