@@ -160,33 +160,7 @@ __device__ __forceinline__ uint64_t value_operand(uint32_t tile) {
 }
 __host__ __device__ constexpr uint32_t value_step(int step) { return step * 16 * 128; }
 
-// The sine (x) and cosine (y) of an angle of at most ANGLE_LIMIT without a branch, so that a thread's
-// several are under way together: Cody and Waite's reduction by n quarter turns, pi/2 in three
-// floats, each step one FMA; polynomials fitted over [-pi/4, pi/4] for the smallest relative error
-// (3.9e-9 and 1.2e-10); the quadrant by n's low bits. At most 1.55 units in the last place off over
-// 20 million angles up to the limit; sincosf is allowed two.
-constexpr float ANGLE_LIMIT = 48000.0f;
-__device__ __forceinline__ float2 sine_and_cosine(float angle) {
-    const float n = rintf(angle * 0.636619772f);
-    float r = fmaf(n, -1.5707963705062866f, angle);
-    r = fmaf(n, 4.371138828673793e-08f, r);
-    r = fmaf(n, 1.7151245100058819e-15f, r);
-    const float z = r * r;
-    float sine = fmaf(z, -0.0001951398007804528f, 0.008332150988280773f);
-    sine = fmaf(z, sine, -0.16666653752326965f);
-    sine = fmaf(r * z, sine, r);
-    float cosine = fmaf(z, 2.4431667043245398e-05f, -0.0013887303648516536f);
-    cosine = fmaf(z, cosine, 0.04166664555668831f);
-    cosine = fmaf(z, cosine, -0.5f);
-    cosine = fmaf(z, cosine, 1.0f);
-    const uint32_t quarter = static_cast<uint32_t>(static_cast<int>(n));
-    const float2 turned = quarter & 1u ? make_float2(cosine, sine) : make_float2(sine, cosine);
-    return make_float2(
-        __uint_as_float(__float_as_uint(turned.x) ^ (quarter << 30 & 0x80000000u)),
-        __uint_as_float(__float_as_uint(turned.y) ^ ((quarter + 1u) << 30 & 0x80000000u)));
-}
-
-// The same of any angle, NaN and infinities among them.
+// sine_and_cosine of any angle, NaN and infinities among them.
 __device__ __noinline__ float2 sine_and_cosine_of_any(float angle) {
     float2 result;
     sincosf(angle, &result.x, &result.y);

@@ -276,3 +276,23 @@ extern "C" int mmh3_b200_batch_items_selftest(const void *query, const void *key
     return mmh3::items_are_independent({query, key, value, output}, tokens, heads, group, head_dim,
                                        batch, *layout);
 }
+
+namespace {
+
+__global__ void sine_and_cosine_kernel(const float *__restrict__ in, float2 *__restrict__ out,
+                                       int angles) {
+    const int index = blockIdx.x * blockDim.x + threadIdx.x;
+    if (index < angles) {
+        out[index] = sm100::sine_and_cosine(in[index]);
+    }
+}
+
+} // namespace
+
+// The sine and cosine of `angles` floats as the fused query RoPE takes them, for angles up to
+// sm100::ANGLE_LIMIT. Device memory; returns a cudaError_t.
+extern "C" int mmh3_b200_sine_and_cosine_selftest(const void *in, void *out, int angles) {
+    sine_and_cosine_kernel<<<(angles + 255) / 256, 256>>>(static_cast<const float *>(in),
+                                                          static_cast<float2 *>(out), angles);
+    return static_cast<int>(cudaGetLastError());
+}

@@ -406,6 +406,63 @@ def test_fused_query_rope_against_float64(element_type, span, head_dim, tokens, 
     assert torch.max(torch.abs(ours.cpu().double() - expected)) <= 2e-2
 
 
+@pytest.mark.parametrize("span", [0.8, 40.0, 1000.0, 47999.0])
+def test_sines_and_cosines_without_a_branch(span):
+    """Against float64, to two units in the last place of the result (what sincosf is allowed): over the
+    span, and next to the multiples of pi/4 in it, where the quadrant changes and where all three parts
+    of pi/2 are needed."""
+    library = load_selftest()
+    generator = torch.Generator().manual_seed(int(span))
+    angles = torch.rand(1 << 21, generator=generator, dtype=torch.float64) * (2 * span) - span
+    turns = torch.randint(-int(span / 0.7854), int(span / 0.7854) + 1, (1 << 20,),
+                          generator=generator).double() * (np.pi / 4)
+    near = turns * (1 + (torch.randint(-3, 4, turns.shape, generator=generator) * 2.0 ** -24))
+    angles = torch.cat([angles, near.clamp(-span, span)]).float().cuda()
+    result = torch.empty((angles.numel(), 2), dtype=torch.float32, device="cuda")
+    assert library.mmh3_b200_sine_and_cosine_selftest(
+        ctypes.c_void_p(angles.data_ptr()), ctypes.c_void_p(result.data_ptr()),
+        angles.numel()) == 0
+    torch.cuda.synchronize()
+    exact = torch.stack([torch.sin(angles.double()), torch.cos(angles.double())], dim=1)
+    unit = torch.exp2(torch.floor(torch.log2(exact.abs().clamp_min(2.0 ** -126))) - 23)
+    # pi/2 in three floats is right to 2^-24 of the third, 1.7e-15 * 6e-8 a quarter turn, at most
+    # 48,000 * 0.64 of them: far below a unit of the smallest sine of a float up to the limit.
+    assert float(((result.double() - exact).abs() / unit).max()) <= 2.0
+
+
+@pytest.mark.parametrize("span", [1000.0, 47900.0])
+@pytest.mark.parametrize("head_dim,pairs", [(64, 32), (64, 20), (128, 64), (128, 33)])
+def test_fused_query_rope_of_large_angles_seen_through_one_key(span, head_dim, pairs):
+    """A key of one dimension at a time reads a rotated query's dimension out of the attention: two
+    keys whose scores differ by the dimension alone, and values of one and zero, give its logistic
+    function."""
+    tokens, heads = 256, 2
+    dims = 24  # heads of the batch: a dimension each
+    generator = torch.Generator().manual_seed(pairs)
+    q = torch.randn((1, tokens, heads, head_dim), generator=generator).half()
+    angles = torch.rand((tokens, pairs), generator=generator) * (2 * span) - span
+    read = torch.linspace(0, head_dim - 1, dims).long()
+    query = q.expand(dims, -1, -1, -1).contiguous()
+    key = torch.zeros((dims, tokens, heads, head_dim)).half()
+    value = torch.zeros_like(key)
+    for item, dimension in enumerate(read.tolist()):
+        key[item, ::2, :, dimension] = 4.0
+        value[item, ::2] = 1.0
+    inner = heads * head_dim
+    layout = attention.make_layout((inner,) * 4, head_stride=(head_dim,) * 4,
+                                   batch_stride=(tokens * inner,) * 4)
+    output = torch.zeros((dims, tokens, heads, head_dim), dtype=torch.float16, device="cuda")
+    attention.attention_roped(1, head_dim, query.cuda(), key.cuda(), value.cuda(), output, tokens,
+                              heads, dims, layout, 0.25, angles.cuda(), pairs, 1e-6)
+    assert attention.take_status() == 0
+    rotated = normalized_rotated(q, angles, pairs, 1e-6, torch.float16)[0].double()
+    expected = torch.sigmoid(rotated[:, :, read]).permute(2, 0, 1)[..., None]
+    # The rotated query may round to the next FP16 value (2^-10 below two, where the logistic passes on
+    # a quarter of it, 2^-9 below four, where it passes on a tenth); P and the output are rounded once
+    # each (2^-11): 1.3e-3 in all.
+    assert float((output.cpu().double() - expected).abs().max()) <= 1.3e-3
+
+
 @pytest.mark.parametrize("element_type", [0, 1])
 def test_heads_of_64_whose_exponentials_come_two_ways(element_type):
     """Two of eight pairs of keys take a polynomial: every key alone in turn holds a row's weight or a
