@@ -79,7 +79,8 @@ struct SharedMemoryOptIn {
 // that the kernel before it has left, then overlap the end of that kernel. It is
 // for the kernels that short calls are made of: INT8/FP8 attention of 2,085 tokens and 56 heads (four
 // kernels) went from 213 us to 204, a causal prompt of 300 tokens (one, behind its like) from 13.0
-// to 12.0. Those of VSA and Sol-Attn, whose calls take milliseconds, are launched as ever.
+// to 12.0. The kernels of VSA and Sol-Attn alone, whose calls take milliseconds, are launched the
+// ordinary way; the pooling pass before them is the inputs pass and is not.
 template <typename... Parameters, typename... Arguments>
 cudaError_t launch_behind(void (*kernel)(Parameters...), dim3 grid, int threads, size_t shared_bytes,
                           cudaStream_t stream, const Arguments &...arguments) {

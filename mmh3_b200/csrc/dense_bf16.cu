@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     const int first_query = query_block * (QUERY_TILES * TILE_M);
     // The last CTA of a sequence may have no row in its second tile. With heads of 64, where the two
     // tiles share an exponential unit that is the bound, it is then left out (eight windows of 1,025
-    // tokens: 105.5 us with it, 102.6 without); with heads of 128 the question costs the long
+    // tokens: 107.9 us with it, 105.3 without); with heads of 128 the question costs the long
     // sequences more (57.9 ms and 58.3 at 66,048 tokens).
     const bool second_tile = DIM != 64 || first_query + TILE_M < tokens;
     const int last_tile = second_tile ? 1 : 0;

@@ -81,7 +81,9 @@ constexpr uint32_t OUTPUT_MMA =
 constexpr float LOG2_224 = 7.807354922057604f;
 constexpr float RESCALE_THRESHOLD = 1.0f;
 // Of every four pairs of probabilities, how many take the polynomial exp2 instead of the MUFU.
-// Measured at L = 66,048 with the integer add below: 0 -> 47.6 ms, 1 -> 50.9 ms, 2 -> 53.0 ms.
+// Measured at L = 66,048 with the integer add below, before the two query tiles took turns at the unit
+// and with a cubic, a shorter polynomial than exp2_polynomial is now: 0 -> 47.6 ms, 1 -> 50.9 ms, 2 ->
+// 53.0 ms.
 constexpr int POLYNOMIAL_PAIRS_OF_4 = 0;
 // An integer score s, |s| < 2^22, becomes the float 1.5 * 2^23 + s by adding these bits to it: an
 // integer add where a conversion would be, which leaves the conversion unit to the exponentials.

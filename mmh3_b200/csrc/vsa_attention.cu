@@ -60,8 +60,9 @@ constexpr uint32_t TMEM_OUTPUT = 128;
 template <bool QUANTIZED> constexpr float RESCALE_LAG = QUANTIZED ? 1.0f : 8.0f;
 constexpr float LOG2_224 = 7.807354922057604f;
 // Of every four pairs of probabilities, how many take the polynomial exp2 instead of the MUFU:
-// none, which at the power cap a layer's worth of launches runs into is 2 % faster than one in
-// four (fewer instructions, a higher clock), as in dense_bf16.cu.
+// none, which at the power cap a layer's worth of launches runs into was 2 % faster than one in
+// four of a cubic, a shorter polynomial than exp2_polynomial is now (fewer instructions, a higher
+// clock), as in dense_bf16.cu.
 constexpr int POLYNOMIAL_PAIRS_OF_4 = 0;
 // In the INT8/FP8 form every exponential takes the MUFU, and an integer score s, |s| < 2^22,
 // becomes the float 1.5 * 2^23 + s by adding these bits to it, as in quantized_attention.cu.
